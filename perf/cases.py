@@ -271,3 +271,84 @@ def tolerance(case):
     if case["kind"] == "two_tile" and case["half"]:
         return {"rel": 1.1e-3, "max": 5e-3}
     return {"rel": 8e-3, "max": 0.2}
+
+
+def _attend(q, k, v, visible, scale):
+    """Attention in 64 bits of [rows, 128] queries over [keys, 128]: row r sees the first visible[r] keys (all: None)."""
+    scores = (q @ k.T).mul_(scale)
+    if visible is not None:
+        seen = torch.arange(k.size(0), device=k.device)[None, :] < visible[:, None]
+        scores.masked_fill_(~seen, -math.inf)
+    lse = scores.logsumexp(-1)
+    return scores.sub_(lse[:, None]).exp_() @ v, lse
+
+
+def _rotate(x, cos, sin):
+    """Rotate-half embedding of x [batch, 1, heads, 128] by the tables' rows cos, sin [batch, 64]."""
+    (lo, hi), (c, s) = x.double().chunk(2, -1), (t.double()[:, None, None, :] for t in (cos, sin))
+    return torch.cat([lo * c - hi * s, hi * c + lo * s], -1)
+
+
+def _exact_decode(q, knew, vnew, kcache, vcache, old, table=None):
+    """O, LSE and the caches after one decode step: the caches keep their type, everything computed is in 64 bits."""
+    out, lse, caches = torch.empty_like(q, dtype=torch.float64), [], [kcache.clone(), vcache.clone()]
+    for b, rows in enumerate(old.tolist()):
+        seen = []
+        for cache, new in zip(caches, (knew, vnew)):
+            if table is None:
+                cache[b, rows], sequence = new[b, 0].to(cache.dtype), cache[b]
+            else:
+                page, row = divmod(rows, cache.size(1))
+                cache[table[b, page], row] = new[b, 0]
+                sequence = cache[table[b, :page + 1].long()].flatten(0, 1)
+            seen.append(torch.cat([sequence[:rows].double(), new[b].double()]))
+        parts = [_attend(q[b, 0, h * GROUP:(h + 1) * GROUP].double(), seen[0][:, h], seen[1][:, h], None, DIM ** -0.5)
+                 for h in range(kcache.size(2))]
+        out[b, 0] = torch.cat([o for o, _ in parts])
+        lse.append(torch.cat([l for _, l in parts]))
+    return [out, torch.stack(lse)[:, :, None], *caches]
+
+
+def _exact_layers(state):
+    plan, cos, sin, old = state["held"]
+    results = []
+    for weights, norms, caches, x, _, _ in plan:
+        y = (x.double() @ weights.double().T).view(x.size(0), 1, 48, DIM)
+        q, k, v = y.split((32, 8, 8), dim=2)
+        at = old.long()
+        q, k = (_rotate(t * (t.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * norm.double(), cos[at], sin[at])
+                for t, norm in ((q, norms[0]), (k, norms[1])))
+        out, lse, kcache, vcache = _exact_decode(q, k, v, *caches, old)
+        results.append([[q, k, v], [kcache, vcache], [out, lse]])
+    return results
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, computed in 64 bits by plain torch."""
+    state = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "layers":
+        return _exact_layers(state)
+    args = state["args"]
+    if kind in ("decode", "paged", "rope"):
+        q, kcache, vcache, knew, vnew, old = args[:6]
+        if kind == "rope":
+            cos, sin = (t[old.long()] for t in state["tables"])
+            q, knew = _rotate(q, cos, sin), _rotate(knew, cos, sin)
+        return _exact_decode(q, knew, vnew, kcache, vcache, old, state.get("table"))
+    q, k, v = args[:3]
+    batch, tokens, heads, _ = q.shape
+    group, causal = heads // k.size(2), kind != "two_tile"
+    out = torch.empty(q.shape, device=q.device, dtype=torch.float64)
+    lse = torch.empty((batch, heads, tokens), device=q.device, dtype=torch.float64)
+    step = 2048
+    for b in range(batch):
+        for h in range(heads):
+            keys, values = (t[b, :, h // group].double() for t in (k, v))
+            for at in range(0, tokens, step):
+                end = min(at + step, tokens)
+                last = end if causal else tokens
+                visible = torch.arange(at + 1, end + 1, device=q.device) if causal else None
+                out[b, at:end, h], lse[b, h, at:end] = _attend(q[b, at:end, h].double(), keys[:last], values[:last],
+                                                               visible, DIM ** -0.5)
+    return [out, lse]
