@@ -101,8 +101,10 @@ int tc_prefill_resources(int device, const int64_t q_strides[3], const int64_t k
  *
  * Replaces `workspace_spec(q,kcache,old_lengths,num_splits,mapping,append) -> int[3]`
  * (tilecadence/cuda/decode/binding.cpp:21, decode.cu:76-83): spec = {splits,
- * splits*B*Hq*128, splits*B*Hq} fp32 elements (zeros when splits == 1). num_splits 0 picks the
- * split count from the SM count; a positive value (<= 128) is used as given.
+ * splits*B*Hq*128, splits*B*Hq} fp32 elements (zeros when splits == 1). A positive num_splits (<= 128) is used as
+ * given for every sequence. 0 leaves it open: a batch of 2 to 64 sequences is then split on the device by the lengths
+ * it finds there (spec names the workspace that this may take; with a workspace that holds only the same number of
+ * splits for every sequence, that is what the call uses), anything else by the SM count.
  */
 int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                              int64_t mapping, int append, int64_t spec[3]);

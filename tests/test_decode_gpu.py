@@ -505,3 +505,40 @@ def test_bound_call_repeats_the_validated_call(ops, gpu_device):
     assert torch.equal(bits(dk.cpu()), bits(want_k)) and torch.equal(bits(dv.cpu()), bits(want_v))
     with pytest.raises(RuntimeError, match="Invalid complete output"):
         ops.bind_forward_out(dq, dk, dv, dkn, dvn, dold, out.float(), lse, *ws, 0, 1, True)
+
+
+@pytest.mark.parametrize("kv_heads,lengths", [
+    (8, [5000, 0]),                                     # everything in one sequence
+    (8, [63, 64, 65, 127, 128]),                        # edges of a tile, fewer tiles than slots
+    (8, [4000, 37, 37, 1900, 0, 250, 3999]),
+    (8, [1000] * 9),                                    # equal lengths
+    (8, [100 * b for b in range(33)]),                  # more than one sequence per lane
+    (8, [64] * 36 + [4000]),                            # as many sequences as CTA slots per KV head
+    (8, [3000] + [10] * 37),                            # more: even splits
+    (1, [9000, 8200] + [130 * b for b in range(62)]),   # one KV head, the largest batch that is split by length
+])
+def test_splits_by_length(gpu_device, kv_heads, lengths):
+    """With the split count left open a batch is split by the lengths on the device; the result agrees with one split per
+    sequence (another order of the same sums: the oracle's bar), with every extra slot idle, and the caches are the same.
+    A workspace of the former size, for even splits, is still accepted."""
+    ops = cuda_runtime.default_ops("decode", 4 * kv_heads)
+    batch, capacity = len(lengths), max(lengths) + 40
+    q, kcache, vcache, knew, vnew = make_case(77, batch, capacity, kv_heads, fill=lengths)
+    old = torch.tensor(lengths, dtype=torch.int32)
+    one_o, one_lse, one_k, one_v, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, num_splits=1)
+    got_o, got_lse, got_k, got_v, spec = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old)
+    oracle.check_outputs(got_o, got_lse, one_o.float(), one_lse)
+    assert torch.equal(bits(got_k), bits(one_k)) and torch.equal(bits(got_v), bits(one_v))
+    again_o, again_lse, _, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, mapping=0)
+    assert torch.equal(bits(got_o), bits(again_o)) and torch.equal(got_lse, again_lse)
+
+    sms = torch.cuda.get_device_properties(gpu_device).multi_processor_count
+    even = max(1, min(sms // (batch * kv_heads), -(-capacity // 64), 128))
+    rows = even * batch * 4 * kv_heads if even > 1 else 0
+    device_tensors = [t.to(gpu_device) for t in (q, kcache, vcache, knew, vnew, old)]
+    out, lse = torch.empty_like(device_tensors[0]), torch.empty((batch, 4 * kv_heads, 1), device=gpu_device)
+    ops.forward_out(*device_tensors, out, lse, torch.empty(rows * 128, device=gpu_device),
+                    torch.empty(rows, device=gpu_device), 0, 1, True)
+    torch.cuda.synchronize()
+    oracle.check_outputs(out.cpu(), lse.cpu(), one_o.float(), one_lse)
+    assert spec[1] >= rows * 128

@@ -51,9 +51,11 @@ constexpr int ring_period(int a, int b) {
     return a / x * b;
 }
 constexpr int kRingPeriod = ring_period(kStages, kGroups);
-// Registers per thread such that AB_DECODE_CTAS_PER_SM CTAs fit the 64 K registers of an SM (allocated per warp
-// in multiples of 8 per thread).
-constexpr int kMaxRegisters = 65536 / (AB_DECODE_CTAS_PER_SM * kThreads) / 8 * 8;
+// Registers per thread such that AB_DECODE_CTAS_PER_SM CTAs fit an SM. Registers belong to the SM's quarters, 16 K
+// each, and are allocated per warp in multiples of 8 per thread: the fullest quarter counts (168 for two CTAs of five
+// warps; at 176 only one CTA was resident).
+constexpr int kWarpsPerQuarter = (AB_DECODE_CTAS_PER_SM * kThreads / 32 + 3) / 4;
+constexpr int kMaxRegisters = 16384 / (32 * kWarpsPerQuarter) / 8 * 8;
 constexpr int kGroup = 4;  // query heads per KV head
 constexpr int kDim = 128;
 constexpr int kMaxSplits = 128;
@@ -96,6 +98,9 @@ constexpr int shared_bytes(bool handoff) {
     return 1024 + kStages * kStageBytes + kBarrierBytes + (handoff ? 0 : kStagingBytes);
 }
 
+constexpr int kSpreadShared = 120 * 1024;  // more than half of an SM's 228 KiB
+static_assert(kSpreadShared >= shared_bytes(false), "room for the schedule");
+
 struct DecodeParams {
     const __nv_bfloat16* q;
     __nv_bfloat16* kcache;
@@ -111,6 +116,9 @@ struct DecodeParams {
     int32_t* tickets;
     int32_t* status;
     int batch, capacity, kv_heads, splits, append, partial;
+    // Splits by length (0: every sequence gets `splits`): the grid holds plan_slots CTAs per KV head, dealt to the
+    // sequences by plan_share; plan_even is the number that puts one CTA on every SM.
+    int plan_slots, plan_even;
     int64_t shard_start;
     float scale, scale_log2;
     uint8_t* peer_blocks[kMaxPeers];  // partial == 2: every rank's exchange block as mapped here
@@ -158,6 +166,106 @@ __device__ __forceinline__ void locate_row(const DecodeParams& p, int b, int slo
         slot = slot_of_b;
         local = row;
     }
+}
+
+// Key tiles of sequence `b` that this launch attends to, from its device-side length. Values outside the contract
+// are clamped so that no address leaves the cache.
+__device__ __forceinline__ int64_t old_length(const DecodeParams& p, int b) {
+    const int64_t length = p.old_lengths[b];
+    return length < 0 ? 0 : length;
+}
+__device__ __forceinline__ int visible_rows(const DecodeParams& p, int64_t old_len) {
+    const int64_t visible = old_len + (p.append ? 1 : 0) - p.shard_start;
+    return int(visible < 0 ? 0 : (visible > p.capacity ? p.capacity : visible));
+}
+
+// Which share of which sequence a CTA of a launch that splits by length works on: sequence b is cut into
+// ceil(tiles_b / size) even shares, at least one. One warp of each CTA works it out from the lengths on the device,
+// every one with the same answer.
+//
+// Why: with the same number of splits for every sequence the longest one sets the time of a ragged batch (one CTA
+// takes a 32 KiB tile in about 0.56 us alone, whatever the others do), while the stream as a whole needs about 112
+// such CTAs to run at the HBM's rate. The estimate that is minimised over 32 sizes, in tile times:
+//   max(longest share, all tiles / 112), and what the shares cost on top:
+//   kMergeCost if any sequence is split (partials, tickets, the last CTA's merge), and if there are more shares
+//   than put one CTA on every SM, kSecondCost and a twelfth of the stream.
+// Equal lengths, and lengths of which none outlasts the stream by what a split costs, need no search: the even split
+// count, or one. Measured (us, even splits before, by length now): 16 paged sequences of 500-8000 rows 72.6 -> 44.5, 24
+// of 300-5000 53.0 -> 34.1, 8 of 200-3333 20.3 -> 15.0; equal lengths pay 0.1 to 0.7 for the look at all of them.
+struct Share {
+    int b, split, splits, first;  // first: slot of the sequence's first share; splits == 0: nothing to do
+    int old_length;
+};
+constexpr float kStreamCtas = 112, kMergeCost = 8, kSecondCost = 2;
+__device__ __forceinline__ Share plan_share(const DecodeParams& p, int slot, int lane) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    const int last = p.batch - 1;
+    // Lanes beyond the batch repeat its last sequence (for the extremes) with a weight of 0 (for the sums).
+    const int64_t old0 = old_length(p, lane < last ? lane : last), old1 = old_length(p, lane + 32 < last ? lane + 32 : last);
+    const uint32_t t0 = uint32_t(visible_rows(p, old0) + kTileN - 1) / kTileN, t1 = uint32_t(visible_rows(p, old1) + kTileN - 1) / kTileN;
+    const bool two = p.batch > 32;
+    const uint32_t total = __reduce_add_sync(kAll, (lane <= last ? t0 : 0u) + (lane + 32 <= last ? t1 : 0u));
+    const uint32_t longest = __reduce_max_sync(kAll, two && t1 > t0 ? t1 : t0);
+    const uint32_t shortest = __reduce_min_sync(kAll, two && t1 < t0 ? t1 : t0);
+    const float stream = float(total) * float(p.kv_heads) * (1.f / kStreamCtas);
+    Share share{};
+    if (longest == shortest || float(longest) <= stream + kMergeCost + kSecondCost) {
+        share.splits = longest == shortest ? p.splits : 1;
+        share.b = share.splits == 1 ? slot : slot / share.splits;
+        share.first = share.b * share.splits;
+        share.split = slot - share.first;
+        if (share.b > last) share.splits = 0;
+    } else {
+        // ceil(tiles / size), at least 1, as a float and without a division or a conversion: adding 2^23 rounds up to
+        // a whole number. Beyond 2^21 tiles it may be off by one, the same in every thread.
+        auto shares = [&](float tiles, float inverse) {
+            const float n = __fadd_ru(fmaf(tiles, inverse, -0.5f * inverse), 8388608.f) - 8388608.f;
+            return fminf(fmaxf(n, 1.f), float(kMaxSplits));
+        };
+        // Lane 0 proposes no splitting, lane 31 the least size that could fit the slots.
+        const float f0 = float(t0), f1 = float(t1), slots = float(p.plan_slots), top = float(longest);
+        const float least = fmaxf(fmaxf(__fdividef(float(total), slots), top * (1.f / kMaxSplits)), 1.f);
+        const float size = lane == 0 ? top : ceilf(fminf(top, least + (top - least) * (float(31 - lane) * (1.f / 31.f))));
+        const float inverse = __frcp_rn(size);
+        float count = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < (two ? 32 : p.batch); ++b) count += shares(__shfl_sync(kAll, f0, b), inverse);
+#pragma unroll 8
+        for (int b = 32; b < p.batch; ++b) count += shares(__shfl_sync(kAll, f1, b - 32), inverse);
+        float estimate = size * (1.f / 32);  // among equals, shorter shares
+        if (count > float(p.plan_even))
+            estimate += fmaxf(size, stream * (13.f / 12)) + kMergeCost + kSecondCost;
+        else
+            estimate += fmaxf(size, stream) + (count > float(p.batch) ? kMergeCost : 0.f);
+        if (count > slots) estimate = INFINITY;  // never lane 0, whose count is the batch
+        // Positive floats are ordered like their bits.
+        const uint32_t best = __reduce_min_sync(kAll, __float_as_uint(estimate));
+        const int chosen = __ffs(int(__ballot_sync(kAll, __float_as_uint(estimate) == best))) - 1;
+        const float cut = __shfl_sync(kAll, inverse, chosen);
+        for (int base = 0; base < p.batch; base += 32) {
+            const int n = base + lane <= last ? int(shares(base == 0 ? f0 : f1, cut)) : 0;
+            int end = n;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const int below = __shfl_up_sync(kAll, end, offset);
+                if (lane >= offset) end += below;
+            }
+            const uint32_t found = __ballot_sync(kAll, slot < share.first + end);
+            if (found) {
+                const int owner = __ffs(int(found)) - 1;
+                share.b = base + owner;
+                share.splits = __shfl_sync(kAll, n, owner);
+                share.first += __shfl_sync(kAll, end - n, owner);
+                share.split = slot - share.first;
+                break;
+            }
+            share.first += __shfl_sync(kAll, end, 31);
+        }
+    }
+    // (int32 on the device, so the length fits again)
+    const int length0 = __shfl_sync(kAll, int(old0), share.b & 31), length1 = __shfl_sync(kAll, int(old1), share.b & 31);
+    share.old_length = share.b < 32 ? length0 : length1;
+    return share;
 }
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory"); }
@@ -240,7 +348,11 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     float* stage_o = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_O_OFFSET_BYTES : 0));
     float* stage_lse = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_LSE_OFFSET_BYTES : 2048));
 
-    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    // A launch that splits by length has its slots in blockIdx.x and, where there are more than one per SM, in two
+    // halves over blockIdx.z: the shares of a coarse cut then occupy the first half of the grid, one per SM.
+    const bool by_length = p.plan_slots > 0;
+    const int kvh = blockIdx.y;
+    __shared__ Share planned;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q_heads = p.kv_heads * kGroup;
 #ifdef TC_TRACE
@@ -269,14 +381,19 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         tc::grid_launch_dependents();
     }
 
-    // Device-side lengths: no host read. Values outside the contract are clamped so that no
-    // address leaves the cache.
-    int64_t old_len = p.old_lengths[b];
-    old_len = old_len < 0 ? 0 : old_len;
-    const int64_t visible_global = old_len + (p.append ? 1 : 0);
-    int64_t visible_local = visible_global - p.shard_start;
-    visible_local = visible_local < 0 ? 0 : (visible_local > p.capacity ? p.capacity : visible_local);
-    const int n_valid = int(visible_local);
+    // Device-side lengths: no host read.
+    if (by_length) {
+        if (warp == kConsumerWarps) {
+            const Share mine = plan_share(p, int(blockIdx.x + blockIdx.z * gridDim.x), lane);
+            if (lane == 0) planned = mine;
+        }
+        __syncthreads();
+    }
+    const Share share = by_length ? planned : Share{int(blockIdx.z), int(blockIdx.x), p.splits, 0, 0};
+    if (share.splits == 0) return;  // more slots than shares
+    const int b = share.b, split = share.split, splits = share.splits;
+    const int64_t old_len = by_length ? share.old_length : old_length(p, b);
+    const int n_valid = visible_rows(p, old_len);
     const int64_t append_local = old_len - p.shard_start;
     const bool do_append = p.append && append_local >= 0 && append_local < p.capacity;
     const int append_row = do_append ? int(append_local) : -1;
@@ -287,11 +404,13 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     }
 
     const int tiles = (n_valid + kTileN - 1) / kTileN;
-    const int tile_begin = int((int64_t(split) * tiles) / p.splits);
-    const int tile_end = int((int64_t(split + 1) * tiles) / p.splits);
+    // (at most 128 splits of 2^24 tiles: 32 bits hold the products, and a 64-bit division would be on the way to the
+    // first load)
+    const int tile_begin = int(uint32_t(split) * uint32_t(tiles) / uint32_t(splits));
+    const int tile_end = int(uint32_t(split + 1) * uint32_t(tiles) / uint32_t(splits));
     const int n_tiles = tile_end - tile_begin;
 
-    __syncthreads();
+    if (!by_length) __syncthreads();
 #ifdef TC_TRACE
     unsigned long long* trace_row = (threadIdx.x == 0 || (warp == kConsumerWarps && lane == 0)) ? g_trace[trace_cta % 1024u] : nullptr;
     if (threadIdx.x == 0) {
@@ -346,7 +465,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             return true;
         };
         if (!p.block_table) {
-            if (lane == 0) {
+            if (tc::elect_one()) {
                 const int ring_early = early_tiles < kStages ? early_tiles : kStages;
                 bool ok = true;
                 int it = 0;
@@ -383,8 +502,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
                 for (int j = 0; j < count && ok; ++j) {
                     const int tile_slot = __shfl_sync(0xffffffffu, slot, j);
                     const int tile_row0 = __shfl_sync(0xffffffffu, local, j);
-                    if (lane == 0) ok = issue_tile(first + j, tile_slot, tile_row0);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    if (tc::elect_one()) ok = issue_tile(first + j, tile_slot, tile_row0);
+                    ok = __all_sync(0xffffffffu, ok);
                 }
             }
         }
@@ -630,16 +749,19 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     const int64_t head_slot = int64_t(b) * p.kv_heads + kvh;  // index of the (batch, KV head) pair
     float4 final_o;
     float final_lse;
-    if (p.splits > 1) {
+    if (splits > 1) {
+        // Partials of a (batch, KV head) pair are `slot_step` slots apart.
+        const int64_t first_slot = by_length ? int64_t(share.first) * p.kv_heads + kvh : head_slot;
+        const int64_t slot_step = by_length ? p.kv_heads : int64_t(p.batch) * p.kv_heads;
         // Vector export of the staged tile: one 16-byte word per thread.
-        const int64_t slot = int64_t(split) * p.batch * p.kv_heads + head_slot;
+        const int64_t slot = first_slot + split * slot_step;
         reinterpret_cast<uint4*>(p.ws_o + slot * (kGroup * kDim))[tid] = reinterpret_cast<const uint4*>(stage_o)[tid];
         if (tid == 0)
             *reinterpret_cast<uint4*>(p.ws_lse + slot * kGroup) = *reinterpret_cast<const uint4*>(stage_lse);
         // The barrier orders every thread's partial stores before thread 0's release; the last
         // arriver's acquire, followed by the second barrier, orders them before the merge loads.
         merge_barrier();
-        if (tid == 0) *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == p.splits - 1;
+        if (tid == 0) *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
         merge_barrier();
         TC_TRACE_POINT(22);
         if (!*flag) return;
@@ -648,9 +770,9 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         // reduce them with shuffles and park the weights in the released terminal K stage; then
         // each lane accumulates its four columns over the splits, with the first batch of partial-O
         // loads already in flight beside the LSE loads.
-        const int64_t stride_lse = int64_t(p.batch) * p.kv_heads * kGroup;
-        const float* lse_base = p.ws_lse + head_slot * kGroup + row;
-        const float4* o_base = reinterpret_cast<const float4*>(p.ws_o + head_slot * (kGroup * kDim) + row * kDim) + col4;
+        const int64_t stride_lse = slot_step * kGroup;
+        const float* lse_base = p.ws_lse + first_slot * kGroup + row;
+        const float4* o_base = reinterpret_cast<const float4*>(p.ws_o + first_slot * (kGroup * kDim) + row * kDim) + col4;
         const int64_t stride_o4 = stride_lse * (kDim / 4);
         float* weights = reinterpret_cast<float*>(terminal_k) + row * kMaxSplits;
         constexpr int kBatch = 20;  // partial-O loads kept in flight per lane
@@ -659,11 +781,11 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
 #pragma unroll
         for (int i = 0; i < kMaxSplits / 32; ++i) {
             const int s = col4 + 32 * i;
-            part_lse[i] = s < p.splits ? __ldcg(lse_base + s * stride_lse) : -INFINITY;
+            part_lse[i] = s < splits ? __ldcg(lse_base + s * stride_lse) : -INFINITY;
         }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)  // first batch goes out with the LSE loads: one L2 round trip
-            if (u < p.splits) v[u] = __ldcg(o_base + u * stride_o4);
+            if (u < splits) v[u] = __ldcg(o_base + u * stride_o4);
         float lse_max = -INFINITY;
 #pragma unroll
         for (int i = 0; i < kMaxSplits / 32; ++i) lse_max = fmaxf(lse_max, part_lse[i]);
@@ -682,15 +804,15 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
         __syncwarp();
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s0 = 0; s0 < p.splits; s0 += kBatch) {
+        for (int s0 = 0; s0 < splits; s0 += kBatch) {
             if (s0 > 0) {
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u)
-                    if (s0 + u < p.splits) v[u] = __ldcg(o_base + (s0 + u) * stride_o4);
+                    if (s0 + u < splits) v[u] = __ldcg(o_base + (s0 + u) * stride_o4);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const float w = s0 + u < p.splits ? weights[s0 + u] : 0.f;
+                const float w = s0 + u < splits ? weights[s0 + u] : 0.f;
                 if (w > 0.f) {  // a split that saw no key may hold anything: never multiply it
                     acc.x = fmaf(w, v[u].x, acc.x);
                     acc.y = fmaf(w, v[u].y, acc.y);
@@ -822,6 +944,33 @@ int auto_splits(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int
     return int(splits);
 }
 
+// Calls that leave the split count open split a batch by length (see plan_share). The number of CTAs per KV head:
+// * where even splits are two or more: as many as those, so that equal lengths leave no CTA idle (with idle CTAs in the
+//   grid, launches that overlap their predecessor's end settle two CTAs on one SM and none on another: 90 us against
+//   81 at four full caches of 32768);
+// * else as many as fill both CTA slots of every SM. Up to one sequence per SM they are kept one to an SM all the
+//   same, for the same reason (16 equal sequences of 2000: 25.9 us, kept apart 23.6, even splits 22.9).
+// Where even splits leave no share longer than a merge costs there is nothing to gain.
+constexpr int kPlanMaxBatch = 64;  // two sequences per lane
+int plan_even(const tc::DeviceInfo& info, int64_t batch, int64_t kv_heads) {
+    const int64_t slots = int64_t(info.sms) / kv_heads;
+    return int(slots > batch ? slots : batch);
+}
+int plan_slots(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits) {
+    const int64_t both = int64_t(info.sms) * AB_DECODE_CTAS_PER_SM / kv_heads;
+    if (num_splits != 0 || batch < 2 || batch > kPlanMaxBatch || batch > both) return 0;
+    const int64_t splits = auto_splits(info, batch, capacity, kv_heads), tiles = (capacity + kTileN - 1) / kTileN;
+    if (tiles <= splits * int64_t(kMergeCost)) return 0;
+    return int(splits > 1 ? splits * batch : both);
+}
+// Splits per sequence that the workspace has to hold: the given or even count, or enough for the slots above.
+int workspace_splits(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
+                     int splits) {
+    const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
+    const int64_t needed = (slots + batch - 1) / batch;
+    return int(needed > splits ? needed : splits);
+}
+
 int check_geometry(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                    int64_t mapping, int append, tc::DeviceInfo* info, int* splits) {
     int status = tc::require_sm100(device, info);
@@ -846,13 +995,19 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
     int device = 0;
     TC_CUDA(cudaGetDevice(&device));
     if (configured_device != device) {
-        TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+        TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadShared));
         configured_device = device;
     }
     cudaLaunchConfig_t config{};
-    config.gridDim = dim3(p.splits, p.kv_heads, p.batch);
+    const int halves = p.plan_slots > 0 && p.splits == 1 ? 2 : 1;
+    // One CTA per SM, by asking for more than half of its shared memory: see plan_slots, and a grid that may start before
+    // its predecessor ends and then finds some SMs emptier than others (four caches of 4096 in a chain of layers: 16.1
+    // -> 15.1 us).
+    const bool spread = p.plan_slots > 0 && (halves == 2 ? p.plan_even > p.batch : p.cache_stable != 0);
+    config.gridDim = p.plan_slots > 0 ? dim3((p.plan_slots + halves - 1) / halves, p.kv_heads, halves)
+                                      : dim3(p.splits, p.kv_heads, p.batch);
     config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = shared;
+    config.dynamicSmemBytes = spread ? kSpreadShared : shared;
     config.stream = stream;
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -941,6 +1096,7 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
                        "every rank's exchange block must be mapped and 16-byte aligned");
         // Every CTA of the grid must be resident at once: a CTA that waits for another rank holds
         // its slot, and the CTAs it indirectly waits for on that rank must never queue behind waiters.
+        // (A launch that splits by length never has more CTAs than fit.)
         TC_REQUIRE(int64_t(splits) * kv_heads * batch <= int64_t(info.sms) * AB_DECODE_CTAS_PER_SM,
                    "peer exchange needs splits*Hkv*B CTAs to be co-resident; lower num_splits");
     }
@@ -967,7 +1123,12 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
     const size_t q_bytes = size_t(rows) * kDim * 2, cache_bytes = size_t(cache_slots) * slot_rows * kv_heads * kDim * 2;
     const size_t new_bytes = size_t(batch) * kv_heads * kDim * 2;
     TC_REQUIRE(cache_bytes <= (size_t(1) << 40), "cache allocation is outside the supported range");
-    const int64_t need_o = splits > 1 ? int64_t(splits) * rows * kDim : 0, need_lse = splits > 1 ? int64_t(splits) * rows : 0;
+    int slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
+    // A workspace that holds the even splits but not the slots is served with the even splits.
+    if (workspace_o_elems < int64_t(slots) * kv_heads * kGroup * kDim || workspace_lse_elems < int64_t(slots) * kv_heads * kGroup)
+        slots = 0;
+    const int64_t need_o = slots > 0 ? int64_t(slots) * kv_heads * kGroup * kDim : splits > 1 ? int64_t(splits) * rows * kDim : 0;
+    const int64_t need_lse = need_o / kDim;
     TC_REQUIRE(workspace_o_elems >= need_o && workspace_lse_elems >= need_lse,
                "Preallocated complete split workspace is too small");
     TC_REQUIRE(!need_o || (workspace_o && workspace_lse), "null split workspace");
@@ -1032,6 +1193,8 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
     p.capacity = int(capacity);
     p.kv_heads = int(kv_heads);
     p.splits = splits;
+    p.plan_slots = slots;
+    p.plan_even = plan_even(info, batch, kv_heads);
     p.append = append ? 1 : 0;
     p.partial = partial;
     p.shard_start = shard_start;
@@ -1164,6 +1327,7 @@ int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_
     if (status != TC_OK) return status;
     TC_REQUIRE(spec, "null spec");
     const int64_t rows = batch * kv_heads * kGroup;
+    splits = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
     spec[0] = splits;
     spec[1] = splits > 1 ? splits * rows * kDim : 0;
     spec[2] = splits > 1 ? splits * rows : 0;
@@ -1220,7 +1384,9 @@ int tc_decode_resources(int device, int64_t batch, int64_t capacity, int64_t kv_
     tc::DeviceGuard guard(device);
     TC_CUDA(guard.status);
     const int64_t rows = batch * kv_heads * kGroup;
-    const int64_t header[12] = {splits, kGroup, kv_heads, kGroup, 1, batch * kv_heads * splits,
+    const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
+    splits = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
+    const int64_t header[12] = {splits, kGroup, kv_heads, kGroup, 1, slots > 0 ? slots * kv_heads : batch * kv_heads * splits,
                                 splits > 1 ? batch * kv_heads : 0, splits > 1 ? splits * rows * kDim : 0,
                                 splits > 1 ? splits * rows : 0, kGroup, kTileN, 1};
     for (int i = 0; i < 12; ++i) values[i] = header[i];
