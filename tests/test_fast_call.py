@@ -1,0 +1,113 @@
+"""The operators' native call path takes exactly the calls that the Python checks take, with the same result."""
+import pytest
+import torch
+
+from oracle import attention as oracle
+from tilecadence_b200 import cuda_runtime
+
+
+def test_native_path_declines_what_it_cannot_take():
+    """Tensors of the host, wrong counts and wrong types: declined with a number, never an exception or a crash."""
+    native = cuda_runtime.fast_call()
+    if native is None:
+        pytest.skip("torch without CUDA")
+    x = torch.zeros(1, 1, 32, 128, dtype=torch.bfloat16)
+    assert native.decode(1, 32, *([x] * 10), 0, 1, True, 0) == -1
+    assert native.prefill(1, 32, *([x] * 7), 0, 1, 0.1, True) == -1
+    assert native.exchange(1, *([x] * 5), False) == -1
+    for name in ("decode", "rope", "indexed", "prefill", "key_split", "exchange"):
+        assert getattr(native, name)() == -1
+        assert getattr(native, name)(*([None] * 17)) == -1
+        assert getattr(native, name)(*(["x"] * 16)) == -1
+
+
+def decode_state(device, batch=2, capacity=256):
+    q, k, v, knew, vnew = (t.to(device) for t in oracle.seeded_normal(
+        5, (batch, 1, 32, 128), (batch, capacity, 8, 128), (batch, capacity, 8, 128), (batch, 1, 8, 128), (batch, 1, 8, 128)))
+    old = torch.arange(100, 100 + batch, dtype=torch.int32, device=device)
+    ops = cuda_runtime.default_ops("decode")
+    spec = ops.workspace_spec(q, k, old, 0, 1, True)
+    results = [torch.empty_like(q), torch.empty((batch, 32, 1), device=device)]
+    workspace = [torch.empty(n, device=device) for n in spec[1:]]
+    return ops, [q, k, v, knew, vnew, old, *results, *workspace, 0, 1, True]
+
+
+def calls(device):
+    ops, args = decode_state(device)
+    table = torch.arange(8, dtype=torch.int32, device=device).view(2, 4)
+    pages = [args[0], args[1].view(8, 64, 8, 128), args[2].view(8, 64, 8, 128), *args[3:]]
+    cos = torch.rand(256, 64, device=device)
+    q, k, v = (t.to(device) for t in oracle.seeded_normal(6, (1, 300, 32, 128), (1, 300, 8, 128), (1, 300, 8, 128)))
+    prefill, out, lse = cuda_runtime.default_ops("prefill"), torch.empty_like(q), torch.empty((1, 32, 300), device=device)
+    none = torch.empty(0, device=device)
+    split = torch.empty(prefill.key_split_workspace_bytes(q), dtype=torch.uint8, device=device)
+    tq = torch.randn(1, 64, 8, 128, device=device, dtype=torch.float16)
+    two = cuda_runtime.default_ops("exchange")
+    return {
+        "decode": (ops.forward_out, args, args[6:8]),
+        "indexed": (lambda *a: ops.indexed_forward_out(*a, block_table=table), pages, args[6:8]),
+        "rope": (lambda *a: ops.rope_forward_out(*a, cos, cos), args, args[6:8]),
+        "prefill": (prefill.forward_out, [q, k, v, out, lse, none, none, 0, 1, 128 ** -0.5, True], [out, lse]),
+        "key_split": (prefill.key_split_forward_out, [q, k, v, out, lse, split, 1, 128 ** -0.5, 2], [out, lse]),
+        "exchange": (two.forward_out, [tq, tq.clone(), tq.clone(), torch.empty_like(tq),
+                                       torch.empty(1, 8, 64, device=device), None, False], None),
+    }
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["decode", "indexed", "rope", "prefill", "key_split", "exchange"])
+def test_both_paths_agree(gpu_device, monkeypatch, name):
+    call, args, results = calls(gpu_device)[name]
+    results = args[3:5] if results is None else results
+    native, taken = cuda_runtime.fast_call(), []
+
+    class Recording:
+        def __getattr__(self, operator):
+            return lambda *a: taken.append(getattr(native, operator)(*a)) or taken[-1]
+
+    monkeypatch.setattr(cuda_runtime, "fast_call", lambda: Recording())
+    call(*args)
+    assert taken == ([2] if name == "key_split" else [0])  # the native path made the call
+    got = [t.clone() for t in results]
+    monkeypatch.setattr(cuda_runtime, "fast_call", lambda: None)
+    call(*args)
+    torch.cuda.synchronize()
+    for a, b in zip(got, results):
+        assert torch.allclose(a, b, atol=1e-2) if name == "key_split" else torch.equal(a, b)
+    # A tensor that the checks refuse is refused with the same words either way: one at a time, another type, a
+    # longer last dimension's stride, autograd.
+    for index, tensor in enumerate(args):
+        if not isinstance(tensor, torch.Tensor) or not tensor.numel():
+            continue
+        bad = [tensor.to(torch.float64), torch.stack([tensor, tensor], -1)[..., 0]]
+        if tensor.is_floating_point():
+            bad.append(tensor.clone().requires_grad_())
+        for wrong in bad:
+            messages = []
+            for path in (native, None):
+                monkeypatch.setattr(cuda_runtime, "fast_call", lambda: path)
+                changed = list(args)
+                changed[index] = wrong
+                try:
+                    call(*changed)
+                    messages.append("")
+                except RuntimeError as error:
+                    messages.append(str(error))
+            assert messages[0] == messages[1]
+    torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+def test_native_path_launches_on_the_current_stream(gpu_device):
+    ops, args = decode_state(gpu_device)
+    graph = torch.cuda.CUDAGraph()
+    stream = torch.cuda.Stream(gpu_device)
+    ops.forward_out(*args)
+    torch.cuda.synchronize()
+    want = args[6].clone()
+    with torch.cuda.graph(graph, stream=stream):  # a launch on another stream would not be captured
+        ops.forward_out(*args)
+    args[6].zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(args[6], want)
