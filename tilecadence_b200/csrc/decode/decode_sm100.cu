@@ -190,8 +190,8 @@ __device__ __forceinline__ int visible_rows(const DecodeParams& p, int64_t old_l
 //   kMergeCost if any sequence is split (partials, tickets, the last CTA's merge), and if there are more shares
 //   than put one CTA on every SM, kSecondCost and a twelfth of the stream.
 // Equal lengths, and lengths of which none outlasts the stream by what a split costs, need no search: the even split
-// count, or one. Measured (us, even splits before, by length now): 16 paged sequences of 500-8000 rows 72.6 -> 44.5, 24
-// of 300-5000 53.0 -> 34.1, 8 of 200-3333 20.3 -> 15.0; equal lengths pay 0.1 to 0.7 for the look at all of them.
+// count, or one. Measured (us, even splits before, by length now): 16 paged sequences of 500-8000 rows 72.7 -> 43.5, 24
+// of 300-5000 52.7 -> 33.7, 8 of 200-3333 20.2 -> 15.1; equal lengths pay 0.1 to 0.8 for the look at all of them.
 struct Share {
     int b, split, splits, first;  // first: slot of the sequence's first share; splits == 0: nothing to do
     int old_length;
@@ -348,8 +348,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     float* stage_o = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_O_OFFSET_BYTES : 0));
     float* stage_lse = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_LSE_OFFSET_BYTES : 2048));
 
-    // A launch that splits by length has its slots in blockIdx.x and, where there are more than one per SM, in two
-    // halves over blockIdx.z: the shares of a coarse cut then occupy the first half of the grid, one per SM.
+    // A launch that splits by length has its slots in blockIdx.x and blockIdx.z, so that equal lengths give every CTA
+    // the place it has in a launch with even splits, and a coarse cut occupies the first CTAs of the grid, one per SM.
     const bool by_length = p.plan_slots > 0;
     const int kvh = blockIdx.y;
     __shared__ Share planned;
@@ -999,13 +999,12 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
         configured_device = device;
     }
     cudaLaunchConfig_t config{};
-    const int halves = p.plan_slots > 0 && p.splits == 1 ? 2 : 1;
+    const int depth = p.plan_slots > 0 ? (p.plan_slots + p.splits - 1) / p.splits : p.batch;
     // One CTA per SM, by asking for more than half of its shared memory: see plan_slots, and a grid that may start before
     // its predecessor ends and then finds some SMs emptier than others (four caches of 4096 in a chain of layers: 16.1
     // -> 15.1 us).
-    const bool spread = p.plan_slots > 0 && (halves == 2 ? p.plan_even > p.batch : p.cache_stable != 0);
-    config.gridDim = p.plan_slots > 0 ? dim3((p.plan_slots + halves - 1) / halves, p.kv_heads, halves)
-                                      : dim3(p.splits, p.kv_heads, p.batch);
+    const bool spread = p.plan_slots > 0 && (p.splits == 1 ? p.plan_even > p.batch : p.cache_stable != 0);
+    config.gridDim = dim3(p.splits, p.kv_heads, depth);
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = spread ? kSpreadShared : shared;
     config.stream = stream;
