@@ -542,3 +542,25 @@ def test_splits_by_length(gpu_device, kv_heads, lengths):
     torch.cuda.synchronize()
     oracle.check_outputs(out.cpu(), lse.cpu(), one_o.float(), one_lse)
     assert spec[1] >= rows * 128
+
+
+def test_exchange_launch_split_by_length_keeps_its_grid_resident(gpu_device):
+    """Twelve sequences, more CTAs than SMs: the launch whose CTAs may wait for other ranks gives the bits of the plain
+    one, which keeps its CTAs one to an SM (asking for more shared memory, also after a look at the resources). With a
+    world of one nobody waits; the host refuses what cannot be resident."""
+    from tilecadence_b200 import sharding
+
+    ops, batch, capacity = cuda_runtime.default_ops("decode"), 12, 1024
+    q, kcache, vcache, knew, vnew = make_case(31, batch, capacity)
+    ops.resources(q.to(gpu_device), kcache.to(gpu_device), torch.zeros(batch, dtype=torch.int32, device=gpu_device), 0, 1, True)
+    old = torch.tensor([1000, 20, 3, 900, 5, 64, 63, 65, 0, 1, 500, 17], dtype=torch.int32)
+    want_o, want_lse, want_k, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old)
+    driver = sharding.ShardedDecode(ops, 0, 1, batch, capacity, gpu_device, exchange="peer")
+    try:
+        dq, dk, dv, dkn, dvn, dold = (t.to(gpu_device) for t in (q, kcache, vcache, knew, vnew, old))
+        out, lse = torch.empty_like(dq), torch.empty((batch, 32, 1), device=gpu_device)
+        driver.step(dq, dk, dv, dkn, dvn, dold, out, lse)
+        torch.cuda.synchronize()
+        assert torch.equal(bits(out.cpu()), bits(want_o)) and torch.equal(bits(dk.cpu()), bits(want_k))
+    finally:
+        driver.close()

@@ -207,10 +207,11 @@ inline bool ranges_overlap(const void* a, size_t a_bytes, const void* b, size_t 
 
 template <typename Kernel>
 inline int kernel_resources(Kernel kernel, int threads, int shared, int64_t* out8) {
-    if (shared >= 48 * 1024)
-        TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
     cudaFuncAttributes attributes{};
     TC_CUDA(cudaFuncGetAttributes(&attributes, kernel));
+    // Only ever raised: a launch may have asked for more, and is not asked again.
+    if (shared >= 48 * 1024 && attributes.maxDynamicSharedSizeBytes < shared)
+        TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
     int active = 0;
     TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, kernel, threads, shared));
     out8[0] = threads;
