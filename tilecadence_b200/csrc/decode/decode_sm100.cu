@@ -1003,7 +1003,8 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
     // One CTA per SM, by asking for more than half of its shared memory: see plan_slots, and a grid that may start before
     // its predecessor ends and then finds some SMs emptier than others (four caches of 4096 in a chain of layers: 16.1
     // -> 15.1 us).
-    const bool spread = p.plan_slots > 0 && (p.splits == 1 ? p.plan_even > p.batch : p.cache_stable != 0);
+    // Never with peers: their CTAs wait for other ranks, so all of the grid's have to be resident at once.
+    const bool spread = !kPeer && p.plan_slots > 0 && (p.splits == 1 ? p.plan_even > p.batch : p.cache_stable != 0);
     config.gridDim = dim3(p.splits, p.kv_heads, depth);
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = spread ? kSpreadShared : shared;
