@@ -103,8 +103,9 @@ int tc_prefill_resources(int device, const int64_t q_strides[3], const int64_t k
  * (tilecadence/cuda/decode/binding.cpp:21, decode.cu:76-83): spec = {splits,
  * splits*B*Hq*128, splits*B*Hq} fp32 elements (zeros when splits == 1). A positive num_splits (<= 128) is used as
  * given for every sequence. 0 leaves it open: a batch of 2 to 64 sequences is then split on the device by the lengths
- * it finds there (spec names the workspace that this may take; with a workspace that holds only the same number of
- * splits for every sequence, that is what the call uses), anything else by the SM count.
+ * it finds there (spec names the workspace that this may take: the partials and, behind the LSEs, 2 elements of ticket
+ * per (sequence, KV head); it needs no initial value. With a workspace that holds only the same number of splits for
+ * every sequence, that is what the call uses), anything else by the SM count.
  */
 int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                              int64_t mapping, int append, int64_t spec[3]);
@@ -117,7 +118,9 @@ int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_
  * new K/V row (bit copy) and keys [0, old_lengths[b]] are attended; without, keys [0, old_lengths[b]).
  * Softmax scale is 128^-0.5 (decode.cu:106). The split partials are merged inside the same launch
  * by the last CTA to finish each (batch, KV head). All ten buffers must be pairwise disjoint
- * (decode.cu:176-177). Calls that share a device must not overlap on the GPU (they share tickets).
+ * (decode.cu:176-177). Calls that share a device must not overlap on the GPU (they share tickets), except calls that
+ * split nothing (num_splits 1) or split by length (their tickets lie in their workspace): those may, each on buffers
+ * and a workspace of its own.
  */
 int tc_decode_forward_out(int device, void* stream, const void* q, void* kcache, void* vcache, const void* knew,
                           const void* vnew, const int32_t* old_lengths, void* out, float* lse,

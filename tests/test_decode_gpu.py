@@ -564,3 +564,41 @@ def test_exchange_launch_split_by_length_keeps_its_grid_resident(gpu_device):
         assert torch.equal(bits(out.cpu()), bits(want_o)) and torch.equal(bits(dk.cpu()), bits(want_k))
     finally:
         driver.close()
+
+
+def test_two_streams_split_by_length_side_by_side(gpu_device):
+    """Batches that even splits leave whole (16 sequences, one split each) share no device state between calls, and
+    neither do they when they are split by length: two streams decode different ragged batches at the same time, each
+    with buffers and a workspace of its own (filled with NaN first), and every result equals the one alone."""
+    ops, batch, capacity, steps = cuda_runtime.default_ops("decode"), 16, 2048, 25
+    work = []
+    for side in range(2):
+        q, kcache, vcache, knew, vnew = (t.to(gpu_device) for t in make_case(91 + side, batch, capacity))
+        old = torch.tensor([(613 * (b + 3 * side) + 17) % (capacity - 1) if b % 5 else capacity - 2 - b for b in range(batch)],
+                           dtype=torch.int32, device=gpu_device)
+        spec = ops.workspace_spec(q, kcache, old, 0, 1, True)
+        ws = [torch.full((n,), float("nan"), device=gpu_device) for n in spec[1:3]]
+        outs = torch.full((steps + 1, *q.shape), float("nan"), device=gpu_device, dtype=torch.bfloat16)
+        lses = torch.full((steps + 1, batch, 32, 1), float("nan"), device=gpu_device)
+        work.append((torch.cuda.Stream(gpu_device), q, kcache, vcache, knew, vnew, old, outs, lses, ws))
+    torch.cuda.synchronize()
+
+    def step(side, index):
+        stream, q, kcache, vcache, knew, vnew, old, outs, lses, ws = work[side]
+        with torch.cuda.stream(stream):
+            ops.forward_out(q, kcache, vcache, knew, vnew, old, outs[index], lses[index], *ws, 0, 1, True)
+
+    for side in range(2):
+        step(side, steps)
+        torch.cuda.synchronize()
+    for index in range(steps):
+        for side in range(2):
+            step(side, index)
+    torch.cuda.synchronize()
+    assert ops.library.device_status(gpu_device.index) == 0
+    for _, q, kcache, vcache, knew, vnew, old, outs, lses, _ in work:
+        alone_o, alone_lse = outs[steps].cpu(), lses[steps].cpu()
+        for index in range(steps):
+            assert torch.equal(bits(outs[index].cpu()), bits(alone_o)) and torch.equal(lses[index].cpu(), alone_lse)
+        want_o, want_lse, _, _ = oracle.decode_step(*(t.cpu() for t in (q, kcache, vcache, knew, vnew, old)))
+        oracle.check_outputs(alone_o, alone_lse, want_o, want_lse)

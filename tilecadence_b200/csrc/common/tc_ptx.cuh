@@ -108,6 +108,11 @@ __device__ __forceinline__ int atomic_add_acq_rel(int* address, int value) {
     asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(address), "r"(value) : "memory");
     return old;
 }
+__device__ __forceinline__ unsigned long long atomic_add_acq_rel(unsigned long long* address, unsigned long long value) {
+    unsigned long long old;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], %2;" : "=l"(old) : "l"(address), "l"(value) : "memory");
+    return old;
+}
 
 // Flag-in-data words for low-latency exchange through another GPU's memory (plain peer stores over
 // NVLink): every aligned 8-byte word carries 4 bytes of payload and a 4-byte flag, and an aligned

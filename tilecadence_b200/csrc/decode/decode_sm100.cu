@@ -61,6 +61,10 @@ constexpr int kDim = 128;
 constexpr int kMaxSplits = 128;
 constexpr int kPrefetchTiles = 12;  // tiles a CTA may prefetch into L2 beyond its shared-memory ring
 constexpr int kEarlyLimitTiles = 32;  // shares longer than this stream nothing ahead of the stream dependency
+// A launch that splits by length counts its finished shares in the caller's workspace, which holds anything at first:
+// a ticket word is this pattern plus the count, and whoever finds another value arms it (see arm_ticket). The pattern's
+// upper half is a NaN with a payload, which no partial result left there by another launch has.
+constexpr unsigned long long kArmed = 0xffa5c3d296e17b00ull;
 constexpr int kStagingBytes = 2304;  // dedicated O/LSE staging when the handoff is disabled
 constexpr int kBarrierBytes = 256;
 // Cross-GPU exchange of per-rank partials (KV sequence sharded over the ranks of one node). Every
@@ -114,6 +118,7 @@ struct DecodeParams {
     float* ws_o;
     float* ws_lse;
     int32_t* tickets;
+    unsigned long long* plan_tickets;  // splits by length: [B * Hkv] in the workspace
     int32_t* status;
     int batch, capacity, kv_heads, splits, append, partial;
     // Splits by length (0: every sequence gets `splits`): the grid holds plan_slots CTAs per KV head, dealt to the
@@ -266,6 +271,15 @@ __device__ __forceinline__ Share plan_share(const DecodeParams& p, int slot, int
     const int length0 = __shfl_sync(kAll, int(old0), share.b & 31), length1 = __shfl_sync(kAll, int(old1), share.b & 31);
     share.old_length = share.b < 32 ? length0 : length1;
     return share;
+}
+
+// Every CTA of a split sequence arms the ticket of its (batch, KV head) once the preceding kernel has completed and
+// long before it takes the ticket: the first one to get there sets the count to zero, the others find the pattern (or
+// lose the exchange to one that does). The last CTA leaves the word armed for the next launch. The words belong to the
+// call's own workspace, so calls on different streams with buffers of their own do not meet here.
+__device__ __forceinline__ void arm_ticket(unsigned long long* ticket) {
+    const unsigned long long found = __ldcg(ticket);
+    if ((found & ~0xffull) != kArmed) atomicCAS(ticket, found, kArmed);
 }
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory"); }
@@ -555,6 +569,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     // Tile `it` belongs to group (n_tiles - 1 - it) % kGroups: the last tile, which lands in stage 0, to group 0,
     // the one before it (stage 1) to group 1. A group's last tile therefore sits in the stage of its own number.
     const int group = warp / kGroupWarps, gw = warp % kGroupWarps;
+    const int64_t head_slot = int64_t(b) * p.kv_heads + kvh;  // index of the (batch, KV head) pair
+    if (by_length && splits > 1 && threadIdx.x == 0) arm_ticket(p.plan_tickets + head_slot);
     const int first_tile = (((n_tiles - 1 - group) % kGroups) + kGroups) % kGroups;
 
     for (int it = first_tile; it < n_tiles; it += kGroups) {
@@ -746,7 +762,6 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     merge_barrier();  // publish the four output rows and their LSE together
     TC_TRACE_POINT(21);
 
-    const int64_t head_slot = int64_t(b) * p.kv_heads + kvh;  // index of the (batch, KV head) pair
     float4 final_o;
     float final_lse;
     if (splits > 1) {
@@ -761,7 +776,9 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         // The barrier orders every thread's partial stores before thread 0's release; the last
         // arriver's acquire, followed by the second barrier, orders them before the merge loads.
         merge_barrier();
-        if (tid == 0) *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
+        if (tid == 0)
+            *flag = by_length ? tc::atomic_add_acq_rel(p.plan_tickets + head_slot, 1ull) == kArmed + uint32_t(splits - 1)
+                              : tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
         merge_barrier();
         TC_TRACE_POINT(22);
         if (!*flag) return;
@@ -827,7 +844,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         final_lse = total > 0.f ? lse_max + logf(total) : -INFINITY;
         // Every split of this head has taken its ticket: a plain store re-arms the counter for the next launch
         // (an atomic exchange would keep this CTA, and with it the end of the kernel, waiting for its return).
-        if (tid == 0) p.tickets[head_slot] = 0;
+        if (tid == 0) {
+            if (by_length) p.plan_tickets[head_slot] = kArmed;
+            else p.tickets[head_slot] = 0;
+        }
     } else {
         final_o = *reinterpret_cast<const float4*>(stage_o + row * kDim + col4 * 4);
         final_lse = stage_lse[row];
@@ -963,7 +983,19 @@ int plan_slots(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int6
     if (tiles <= splits * int64_t(kMergeCost)) return 0;
     return int(splits > 1 ? splits * batch : both);
 }
-// Splits per sequence that the workspace has to hold: the given or even count, or enough for the slots above.
+// FP32 elements of the workspace that a launch with `slots` slots uses: the partial O and LSE of every slot, behind
+// the LSEs one 8-byte ticket per (batch, KV head).
+int64_t plan_o_elems(int64_t slots, int64_t kv_heads) { return slots * kv_heads * kGroup * kDim; }
+int64_t plan_lse_elems(int64_t slots, int64_t batch, int64_t kv_heads) { return slots * kv_heads * kGroup + (slots > 0 ? batch * kv_heads * 2 : 0); }
+// What tc_decode_workspace_spec and tc_decode_resources report: room for either kind of launch.
+void workspace_elems(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
+                     int splits, int64_t* o_elems, int64_t* lse_elems) {
+    const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
+    const int64_t even_lse = splits > 1 ? splits * batch * kv_heads * kGroup : 0;
+    const int64_t plan_o = plan_o_elems(slots, kv_heads), plan_lse = plan_lse_elems(slots, batch, kv_heads);
+    *o_elems = plan_o > even_lse * kDim ? plan_o : even_lse * kDim;
+    *lse_elems = plan_lse > even_lse ? plan_lse : even_lse;
+}
 int workspace_splits(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                      int splits) {
     const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
@@ -1124,11 +1156,10 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
     const size_t new_bytes = size_t(batch) * kv_heads * kDim * 2;
     TC_REQUIRE(cache_bytes <= (size_t(1) << 40), "cache allocation is outside the supported range");
     int slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
-    // A workspace that holds the even splits but not the slots is served with the even splits.
-    if (workspace_o_elems < int64_t(slots) * kv_heads * kGroup * kDim || workspace_lse_elems < int64_t(slots) * kv_heads * kGroup)
-        slots = 0;
-    const int64_t need_o = slots > 0 ? int64_t(slots) * kv_heads * kGroup * kDim : splits > 1 ? int64_t(splits) * rows * kDim : 0;
-    const int64_t need_lse = need_o / kDim;
+    // A workspace that holds the even splits but not the slots and their tickets is served with the even splits.
+    if (workspace_o_elems < plan_o_elems(slots, kv_heads) || workspace_lse_elems < plan_lse_elems(slots, batch, kv_heads)) slots = 0;
+    const int64_t need_o = slots > 0 ? plan_o_elems(slots, kv_heads) : splits > 1 ? int64_t(splits) * rows * kDim : 0;
+    const int64_t need_lse = slots > 0 ? plan_lse_elems(slots, batch, kv_heads) : need_o / kDim;
     TC_REQUIRE(workspace_o_elems >= need_o && workspace_lse_elems >= need_lse,
                "Preallocated complete split workspace is too small");
     TC_REQUIRE(!need_o || (workspace_o && workspace_lse), "null split workspace");
@@ -1188,6 +1219,7 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
     p.ws_o = workspace_o;
     p.ws_lse = workspace_lse;
     p.tickets = scratch.tickets;
+    if (slots > 0) p.plan_tickets = reinterpret_cast<unsigned long long*>(workspace_lse + int64_t(slots) * kv_heads * kGroup);
     p.status = scratch.status;
     p.batch = int(batch);
     p.capacity = int(capacity);
@@ -1326,11 +1358,8 @@ int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_
     int status = check_geometry(device, batch, capacity, kv_heads, num_splits, mapping, append, &info, &splits);
     if (status != TC_OK) return status;
     TC_REQUIRE(spec, "null spec");
-    const int64_t rows = batch * kv_heads * kGroup;
-    splits = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
-    spec[0] = splits;
-    spec[1] = splits > 1 ? splits * rows * kDim : 0;
-    spec[2] = splits > 1 ? splits * rows : 0;
+    workspace_elems(info, batch, capacity, kv_heads, num_splits, splits, &spec[1], &spec[2]);
+    spec[0] = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
     return TC_OK;
 }
 
@@ -1383,12 +1412,12 @@ int tc_decode_resources(int device, int64_t batch, int64_t capacity, int64_t kv_
     TC_REQUIRE(values && count && capacity_values >= 34, "resources needs room for 34 values");
     tc::DeviceGuard guard(device);
     TC_CUDA(guard.status);
-    const int64_t rows = batch * kv_heads * kGroup;
     const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
+    int64_t o_elems, lse_elems;
+    workspace_elems(info, batch, capacity, kv_heads, num_splits, splits, &o_elems, &lse_elems);
     splits = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
     const int64_t header[12] = {splits, kGroup, kv_heads, kGroup, 1, slots > 0 ? slots * kv_heads : batch * kv_heads * splits,
-                                splits > 1 ? batch * kv_heads : 0, splits > 1 ? splits * rows * kDim : 0,
-                                splits > 1 ? splits * rows : 0, kGroup, kTileN, 1};
+                                splits > 1 ? batch * kv_heads : 0, o_elems, lse_elems, kGroup, kTileN, 1};
     for (int i = 0; i < 12; ++i) values[i] = header[i];
     status = mapping == 1 ? tc::kernel_resources(&decode_splitkv_kernel<true, false>, kThreads, shared_bytes(true), values + 12)
                           : tc::kernel_resources(&decode_splitkv_kernel<false, false>, kThreads, shared_bytes(false), values + 12);
