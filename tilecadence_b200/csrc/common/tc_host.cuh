@@ -205,13 +205,26 @@ inline bool ranges_overlap(const void* a, size_t a_bytes, const void* b, size_t 
     return x < y + b_bytes && y < x + a_bytes;
 }
 
+// The dynamic shared memory that launches of `kernel` on the current device may ask for is at least `shared` from here
+// on. The limit belongs to the whole process: it is only ever raised, and looking and raising are one step for all
+// threads, because a launch that has raised it once does not ask again. Every use of the attribute goes through here.
 template <typename Kernel>
-inline int kernel_resources(Kernel kernel, int threads, int shared, int64_t* out8) {
+inline int raise_shared_limit(Kernel kernel, int shared) {
+    static std::mutex lock;
+    std::lock_guard<std::mutex> guard(lock);
     cudaFuncAttributes attributes{};
     TC_CUDA(cudaFuncGetAttributes(&attributes, kernel));
-    // Only ever raised: a launch may have asked for more, and is not asked again.
-    if (shared >= 48 * 1024 && attributes.maxDynamicSharedSizeBytes < shared)
+    if (attributes.maxDynamicSharedSizeBytes < shared)
         TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+    return TC_OK;
+}
+
+template <typename Kernel>
+inline int kernel_resources(Kernel kernel, int threads, int shared, int64_t* out8) {
+    int status = raise_shared_limit(kernel, shared);
+    if (status != TC_OK) return status;
+    cudaFuncAttributes attributes{};
+    TC_CUDA(cudaFuncGetAttributes(&attributes, kernel));
     int active = 0;
     TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, kernel, threads, shared));
     out8[0] = threads;

@@ -1027,7 +1027,8 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
     int device = 0;
     TC_CUDA(cudaGetDevice(&device));
     if (configured_device != device) {
-        TC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadShared));
+        const int status = tc::raise_shared_limit(kernel, kSpreadShared);
+        if (status != TC_OK) return status;
         configured_device = device;
     }
     cudaLaunchConfig_t config{};

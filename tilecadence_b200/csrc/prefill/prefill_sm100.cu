@@ -1312,10 +1312,10 @@ int launch(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& 
     int device = 0;
     TC_CUDA(cudaGetDevice(&device));
     if (configured_device != device) {
-        TC_CUDA(cudaFuncSetAttribute(&prefill_kernel<kHandoff, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     shared_bytes(kHandoff)));
-        TC_CUDA(cudaFuncSetAttribute(&prefill_rowblock_kernel<kHandoff, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     rowblock_shared_bytes(kHandoff)));
+        int status = tc::raise_shared_limit(&prefill_kernel<kHandoff, kSplit>, shared_bytes(kHandoff));
+        if (status == TC_OK)
+            status = tc::raise_shared_limit(&prefill_rowblock_kernel<kHandoff, kSplit>, rowblock_shared_bytes(kHandoff));
+        if (status != TC_OK) return status;
         configured_device = device;
     }
     // Either way the shared memory and the tensor memory of a CTA leave room for one CTA per SM.

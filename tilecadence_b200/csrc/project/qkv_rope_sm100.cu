@@ -362,7 +362,8 @@ int tc_qkv_rope_forward_out_flags(int device, void* stream, const void* x, const
 
     static thread_local int configured_device = -1, configured_shared = 0;
     if (configured_device != device || configured_shared < shared) {
-        TC_CUDA(cudaFuncSetAttribute(qkv_rope_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+        status = tc::raise_shared_limit(&qkv_rope_kernel, shared);
+        if (status != TC_OK) return status;
         configured_device = device;
         configured_shared = shared;
     }
