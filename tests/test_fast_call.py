@@ -21,6 +21,14 @@ def test_native_path_declines_what_it_cannot_take():
         assert getattr(native, name)(*(["x"] * 16)) == -1
 
 
+def test_nothing_of_a_tensor_is_read_without_the_interpreter_lock():
+    """Another thread may resize a tensor as soon as the lock is released: what the launch gets are numbers read before."""
+    source = (cuda_runtime.PACKAGE_ROOT / "host" / "fast_call.cpp").read_text()
+    released = source.split("Py_BEGIN_ALLOW_THREADS")[1:]
+    assert len(released) == 1 and released[0].split("Py_END_ALLOW_THREADS")[0].split() == ["status", "=", "function(arguments...);"]
+    assert "without_gil([" not in source  # a closure would read its captures after the release
+
+
 def decode_state(device, batch=2, capacity=256):
     q, k, v, knew, vnew = (t.to(device) for t in oracle.seeded_normal(
         5, (batch, 1, 32, 128), (batch, capacity, 8, 128), (batch, capacity, 8, 128), (batch, 1, 8, 128), (batch, 1, 8, 128)))

@@ -11,6 +11,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <initializer_list>
+#include <type_traits>
 
 #include "tilecadence_b200.h"
 
@@ -52,12 +53,15 @@ bool truth(PyObject* object, bool* out) {
 
 void* address(const at::Tensor& tensor) { return tensor.numel() ? tensor.data_ptr() : nullptr; }
 
-// As ctypes does for a foreign function: other Python threads may run while the launch is made.
-template <class Call>
-int without_gil(Call call) {
+// As ctypes does for a foreign function: other Python threads may run while the launch is made. Addresses, sizes and
+// strides therefore arrive as numbers, read while the GIL was still held: another thread may resize or re-point a tensor
+// from here on.
+template <class Function, class... Arguments>
+int without_gil(Function function, Arguments... arguments) {
+    static_assert((... && !std::is_same_v<std::remove_cv_t<std::remove_pointer_t<Arguments>>, at::Tensor>), "no tensors");
     int status;
     Py_BEGIN_ALLOW_THREADS
-    status = call();
+    status = function(arguments...);
     Py_END_ALLOW_THREADS
     return status;
 }
@@ -108,12 +112,11 @@ int decode_call(PyObject* const* a, Py_ssize_t n) {
     int64_t heads, flags;
     if (n != 16 || !whole(a[1], &heads) || !whole(a[15], &flags) || !d.read(a + 2, heads, false)) return kNotTaken;
     const auto function = entry<decltype(&tc_decode_forward_out_flags)>(a[0]);
-    return without_gil([&] {
-        return function(d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew), address(*d.vnew),
-                        static_cast<const int32_t*>(address(*d.old)), address(*d.out), static_cast<float*>(address(*d.lse)),
-                        static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(), static_cast<float*>(address(*d.ws_lse)),
-                        d.ws_lse->numel(), d.batch, d.k->size(1), d.heads, d.splits, d.mapping, d.append, flags);
-    });
+    return without_gil(function, d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew),
+                       address(*d.vnew), static_cast<const int32_t*>(address(*d.old)), address(*d.out),
+                       static_cast<float*>(address(*d.lse)), static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(),
+                       static_cast<float*>(address(*d.ws_lse)), d.ws_lse->numel(), d.batch, d.k->size(1), d.heads,
+                       d.splits, d.mapping, d.append, flags);
 }
 
 // (address of tc_decode_rope_forward_out, q heads, the 13 arguments, cos, sin)
@@ -127,13 +130,12 @@ int rope_call(PyObject* const* a, Py_ssize_t n) {
             !t->is_contiguous() || t->sizes() != cos->sizes())
             return kNotTaken;
     const auto function = entry<decltype(&tc_decode_rope_forward_out)>(a[0]);
-    return without_gil([&] {
-        return function(d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew), address(*d.vnew),
-                        static_cast<const int32_t*>(address(*d.old)), address(*d.out), static_cast<float*>(address(*d.lse)),
-                        static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(), static_cast<float*>(address(*d.ws_lse)),
-                        d.ws_lse->numel(), d.batch, d.k->size(1), d.heads, d.splits, d.mapping, d.append,
-                        static_cast<const float*>(address(*cos)), static_cast<const float*>(address(*sin)), cos->size(0));
-    });
+    return without_gil(function, d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew),
+                       address(*d.vnew), static_cast<const int32_t*>(address(*d.old)), address(*d.out),
+                       static_cast<float*>(address(*d.lse)), static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(),
+                       static_cast<float*>(address(*d.ws_lse)), d.ws_lse->numel(), d.batch, d.k->size(1), d.heads,
+                       d.splits, d.mapping, d.append, static_cast<const float*>(address(*cos)),
+                       static_cast<const float*>(address(*sin)), cos->size(0));
 }
 
 // (address of tc_decode_indexed_forward_out, q heads, the 13 arguments, block_table or None, cache_batch_idx or None)
@@ -148,14 +150,12 @@ int indexed_call(PyObject* const* a, Py_ssize_t n) {
         return kNotTaken;
     const auto function = entry<decltype(&tc_decode_indexed_forward_out)>(a[0]);
     const int32_t* table = static_cast<const int32_t*>(address(*index));
-    return without_gil([&] {
-        return function(d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew), address(*d.vnew),
-                        static_cast<const int32_t*>(address(*d.old)), address(*d.out), static_cast<float*>(address(*d.lse)),
-                        static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(), static_cast<float*>(address(*d.ws_lse)),
-                        d.ws_lse->numel(), d.batch, d.k->size(0), d.k->size(1), d.heads, d.splits, d.mapping, d.append,
-                        paged ? table : nullptr, paged ? index->stride(0) : 0, paged ? index->size(1) : 0,
-                        paged ? nullptr : table);
-    });
+    return without_gil(function, d.device, d.stream, address(*d.q), address(*d.k), address(*d.v), address(*d.knew),
+                       address(*d.vnew), static_cast<const int32_t*>(address(*d.old)), address(*d.out),
+                       static_cast<float*>(address(*d.lse)), static_cast<float*>(address(*d.ws_o)), d.ws_o->numel(),
+                       static_cast<float*>(address(*d.ws_lse)), d.ws_lse->numel(), d.batch, d.k->size(0), d.k->size(1),
+                       d.heads, d.splits, d.mapping, d.append, paged ? table : nullptr, paged ? index->stride(0) : 0,
+                       paged ? index->size(1) : 0, paged ? nullptr : table);
 }
 
 // q, k, v, out, lse of the prefill operators.
@@ -208,11 +208,9 @@ int prefill_call(PyObject* const* a, Py_ssize_t n) {
         return kNotTaken;
     const double scale = PyFloat_AS_DOUBLE(a[11]);
     const auto function = entry<decltype(&tc_prefill_forward_out)>(a[0]);
-    return without_gil([&] {
-        return function(p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1], address(*p.v),
-                        p.strides[2], address(*p.out), static_cast<float*>(address(*p.lse)), 0, 0, p.batch, p.tokens, p.heads,
-                        splits, mapping, scale, 1);
-    });
+    return without_gil(function, p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1],
+                       address(*p.v), p.strides[2], address(*p.out), static_cast<float*>(address(*p.lse)), 0, 0, p.batch,
+                       p.tokens, p.heads, splits, mapping, scale, 1);
 }
 
 // (address of tc_prefill_key_split_forward_out, q heads, q, k, v, out, lse, workspace, mapping, scale, key_splits).
@@ -227,11 +225,10 @@ int key_split_call(PyObject* const* a, Py_ssize_t n) {
         return kNotTaken;
     const double scale = PyFloat_AS_DOUBLE(a[9]);
     const auto function = entry<decltype(&tc_prefill_key_split_forward_out)>(a[0]);
-    const int status = without_gil([&] {
-        return function(p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1], address(*p.v),
-                        p.strides[2], address(*p.out), static_cast<float*>(address(*p.lse)), address(*workspace),
-                        workspace->numel(), p.batch, p.tokens, p.heads, mapping, scale, key_splits, &used);
-    });
+    const int status = without_gil(function, p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1],
+                                   address(*p.v), p.strides[2], address(*p.out), static_cast<float*>(address(*p.lse)),
+                                   address(*workspace), workspace->numel(), p.batch, p.tokens, p.heads, mapping, scale,
+                                   key_splits, &used);
     return status == TC_OK ? int(used) : kNotTaken;
 }
 
@@ -253,10 +250,8 @@ int exchange_call(PyObject* const* a, Py_ssize_t n) {
     const int device = q->device().index();
     void* stream = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
     const auto function = entry<decltype(&tc_exchange_forward_out)>(a[0]);
-    return without_gil([&] {
-        return function(device, stream, address(*q), address(*k), address(*v), address(*out), static_cast<float*>(address(*lse)),
-                        batch, heads, type == at::kHalf, causal);
-    });
+    return without_gil(function, device, stream, address(*q), address(*k), address(*v), address(*out),
+                       static_cast<float*>(address(*lse)), batch, heads, type == at::kHalf, causal);
 }
 
 template <int (*call)(PyObject* const*, Py_ssize_t)>
