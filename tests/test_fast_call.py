@@ -21,6 +21,41 @@ def test_native_path_declines_what_it_cannot_take():
         assert getattr(native, name)(*(["x"] * 16)) == -1
 
 
+@pytest.mark.parametrize("fault", ["no compiler", "compiler fails", "broken library"])
+def test_operators_work_without_the_native_path(monkeypatch, tmp_path, fault):
+    """Where the native path can be neither found nor built, the operators say so once and go through their checks."""
+    if cuda_runtime.fast_call() is None:
+        pytest.skip("torch without CUDA")
+    library = next(cuda_runtime.BUILD_DIR.glob("tc_fast_call_*.so"))
+    monkeypatch.setattr(cuda_runtime, "BUILD_DIR", tmp_path)
+    if fault == "no compiler":
+        monkeypatch.setattr(cuda_runtime.shutil, "which", lambda name: None)
+    elif fault == "compiler fails":
+        monkeypatch.setattr(cuda_runtime.subprocess, "run",
+                            lambda *a, **k: cuda_runtime.subprocess.CompletedProcess(a, 1, "", "no headers"))
+    else:
+        for path in cuda_runtime.PACKAGE_ROOT.glob(f"_build/{library.name[:13]}*.so"):
+            (tmp_path / path.name).write_bytes(b"not a library")
+
+    class Prebuilt:
+        addresses = {"tc_decode_forward_out_flags": 1}
+
+        def has(self, prefix):
+            return prefix == "tc_decode_"
+
+    x = torch.zeros(1, 1, 32, 128, dtype=torch.bfloat16)
+    cuda_runtime.fast_call.cache_clear()
+    try:
+        with pytest.warns(RuntimeWarning, match="checks in Python") as said:
+            ops = cuda_runtime.ops_for(Prebuilt())
+            for _ in range(2):
+                with pytest.raises(RuntimeError, match="must be CUDA on the same device"):
+                    ops.forward_out(*([x] * 10), 0, 1, True)
+        assert len(said) == 1
+    finally:
+        cuda_runtime.fast_call.cache_clear()
+
+
 def test_nothing_of_a_tensor_is_read_without_the_interpreter_lock():
     """Another thread may resize a tensor as soon as the lock is released: what the launch gets are numbers read before."""
     source = (cuda_runtime.PACKAGE_ROOT / "host" / "fast_call.cpp").read_text()
