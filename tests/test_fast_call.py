@@ -1,4 +1,6 @@
 """The operators' native call path takes exactly the calls that the Python checks take, with the same result."""
+import ctypes
+
 import pytest
 import torch
 
@@ -75,17 +77,19 @@ def decode_state(device, batch=2, capacity=256):
     return ops, [q, k, v, knew, vnew, old, *results, *workspace, 0, 1, True]
 
 
-def calls(device):
-    ops, args = decode_state(device)
+def calls(device, made_by=cuda_runtime.default_ops):
+    """Operator, arguments and results of one call each; the operator objects called come from ``made_by``."""
+    _, args = decode_state(device)
+    ops = made_by("decode")
     table = torch.arange(8, dtype=torch.int32, device=device).view(2, 4)
     pages = [args[0], args[1].view(8, 64, 8, 128), args[2].view(8, 64, 8, 128), *args[3:]]
     cos = torch.rand(256, 64, device=device)
     q, k, v = (t.to(device) for t in oracle.seeded_normal(6, (1, 300, 32, 128), (1, 300, 8, 128), (1, 300, 8, 128)))
-    prefill, out, lse = cuda_runtime.default_ops("prefill"), torch.empty_like(q), torch.empty((1, 32, 300), device=device)
+    prefill, out, lse = made_by("prefill"), torch.empty_like(q), torch.empty((1, 32, 300), device=device)
     none = torch.empty(0, device=device)
-    split = torch.empty(prefill.key_split_workspace_bytes(q), dtype=torch.uint8, device=device)
+    split = torch.empty(cuda_runtime.default_ops("prefill").key_split_workspace_bytes(q), dtype=torch.uint8, device=device)
     tq = torch.randn(1, 64, 8, 128, device=device, dtype=torch.float16)
-    two = cuda_runtime.default_ops("exchange")
+    two = made_by("exchange")
     return {
         "decode": (ops.forward_out, args, args[6:8]),
         "indexed": (lambda *a: ops.indexed_forward_out(*a, block_table=table), pages, args[6:8]),
@@ -138,6 +142,26 @@ def test_both_paths_agree(gpu_device, monkeypatch, name):
                     messages.append(str(error))
             assert messages[0] == messages[1]
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["decode", "indexed", "rope", "prefill", "key_split", "exchange"])
+def test_a_call_that_fails_in_the_entry_point_is_made_once(gpu_device, name):
+    """An error of the C ABI is raised from the native path; the call is not made again through ctypes. The entry point
+    here is a stand-in that counts and launches nothing."""
+    made = []
+    stand_in = ctypes.CFUNCTYPE(ctypes.c_int)(lambda: made.append("native") or 2)
+    real = cuda_runtime.default_library()
+
+    class Failing:
+        path, handle, symbols, fail, call = real.path, real.handle, real.symbols, cuda_runtime.Library.fail, cuda_runtime.Library.call
+        addresses = dict.fromkeys(real.addresses, ctypes.cast(stand_in, ctypes.c_void_p).value)
+        functions = dict.fromkeys(real.functions, lambda *a: made.append("ctypes") or 2)
+
+    operator, args, _ = calls(gpu_device, lambda phase: cuda_runtime.ops_for(Failing(), phase))[name]
+    with pytest.raises(RuntimeError, match=r"^tc_[a-z_]*_out: .*status 2"):
+        operator(*args)
+    assert made == ["native"]
 
 
 @pytest.mark.gpu

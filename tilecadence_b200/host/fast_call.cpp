@@ -4,9 +4,10 @@
 // Why: a decode step on a short cache takes 6 us on the GPU, while the same checks through tensor attributes and the
 // argument conversion of ctypes took 14 to 16 us of host time per call, so that every small call was bound by them.
 //
-// Each function returns 0 when the call has been made and succeeded. Anything else (a check that fails, an argument of
-// another type than expected, a tensor subclass, an error of the C ABI) returns non-zero and the Python operator goes
-// through its own checks and call, which raise what they always raised. Nothing is kept between calls.
+// Each function returns -1 when it does not take the call (a check that fails, an argument of another type than
+// expected, a tensor subclass): the Python operator then goes through its own checks and call, which raise what they
+// always raised. Otherwise the call has been made, once, and the result is 16 times the status of the C ABI plus what
+// the call returns (0, or the number of key splits). Nothing is kept between calls.
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -63,7 +64,7 @@ int without_gil(Function function, Arguments... arguments) {
     Py_BEGIN_ALLOW_THREADS
     status = function(arguments...);
     Py_END_ALLOW_THREADS
-    return status;
+    return status * 16;
 }
 
 template <class Function>
@@ -214,7 +215,7 @@ int prefill_call(PyObject* const* a, Py_ssize_t n) {
 }
 
 // (address of tc_prefill_key_split_forward_out, q heads, q, k, v, out, lse, workspace, mapping, scale, key_splits).
-// Returns the number of key splits used.
+// Returns the number of key splits used with the status.
 int key_split_call(PyObject* const* a, Py_ssize_t n) {
     Prefill p;
     int64_t heads, mapping, key_splits, used = 0;
@@ -225,11 +226,11 @@ int key_split_call(PyObject* const* a, Py_ssize_t n) {
         return kNotTaken;
     const double scale = PyFloat_AS_DOUBLE(a[9]);
     const auto function = entry<decltype(&tc_prefill_key_split_forward_out)>(a[0]);
-    const int status = without_gil(function, p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1],
+    const int result = without_gil(function, p.device, p.stream, address(*p.q), p.strides[0], address(*p.k), p.strides[1],
                                    address(*p.v), p.strides[2], address(*p.out), static_cast<float*>(address(*p.lse)),
                                    address(*workspace), workspace->numel(), p.batch, p.tokens, p.heads, mapping, scale,
                                    key_splits, &used);
-    return status == TC_OK ? int(used) : kNotTaken;
+    return result + int(used);
 }
 
 // (address of tc_exchange_forward_out, q, k, v, out, lse, causal)
