@@ -602,3 +602,25 @@ def test_two_streams_split_by_length_side_by_side(gpu_device):
             assert torch.equal(bits(outs[index].cpu()), bits(alone_o)) and torch.equal(lses[index].cpu(), alone_lse)
         want_o, want_lse, _, _ = oracle.decode_step(*(t.cpu() for t in (q, kcache, vcache, knew, vnew, old)))
         oracle.check_outputs(alone_o, alone_lse, want_o, want_lse)
+
+
+@pytest.mark.parametrize("batch,capacity,splits", [(4, 4096, 4), (16, 2048, 1), (37, 1024, 1), (2, 300, 5)])
+def test_the_workspace_spec_still_names_the_split_count(gpu_device, batch, capacity, splits):
+    """spec[0] and resources()[0] are the number of splits that every sequence gets for the SM count, whatever the
+    workspace holds beside them: handed back as num_splits it is the launch with even splits, bit for bit."""
+    ops = cuda_runtime.default_ops("decode")
+    case = make_case(17, batch, capacity)
+    old = torch.tensor([(777 * b) % (capacity - 1) for b in range(batch)], dtype=torch.int32)
+    q, kcache, vcache, knew, vnew, dold = [t.to(gpu_device) for t in (*case, old)]
+    spec = ops.workspace_spec(q, kcache, dold, 0, 1, True)
+    resources = ops.resources(q, kcache, dold, 0, 1, True)
+    even = ops.workspace_spec(q, kcache, dold, splits, 1, True)
+    assert spec[0] == resources[0] == splits and resources[7:9] == spec[1:]
+    assert spec[1] >= even[1] and spec[2] >= even[2] and ops.indexed_workspace_spec(batch, capacity, 8, gpu_device.index) == spec
+    results = []
+    for num_splits, workspace in ((spec[0], spec), (0, even)):
+        out, lse = torch.empty_like(q), torch.empty((batch, 32, 1), device=gpu_device)
+        ops.forward_out(q, kcache, vcache, knew, vnew, dold, out, lse,
+                        *(torch.full((n,), float("nan"), device=gpu_device) for n in workspace[1:]), num_splits, 1, True)
+        results.append((out.cpu(), lse.cpu()))
+    assert torch.equal(bits(results[0][0]), bits(results[1][0])) and torch.equal(results[0][1], results[1][1])

@@ -996,12 +996,6 @@ void workspace_elems(const tc::DeviceInfo& info, int64_t batch, int64_t capacity
     *o_elems = plan_o > even_lse * kDim ? plan_o : even_lse * kDim;
     *lse_elems = plan_lse > even_lse ? plan_lse : even_lse;
 }
-int workspace_splits(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
-                     int splits) {
-    const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
-    const int64_t needed = (slots + batch - 1) / batch;
-    return int(needed > splits ? needed : splits);
-}
 
 int check_geometry(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                    int64_t mapping, int append, tc::DeviceInfo* info, int* splits) {
@@ -1359,8 +1353,8 @@ int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_
     int status = check_geometry(device, batch, capacity, kv_heads, num_splits, mapping, append, &info, &splits);
     if (status != TC_OK) return status;
     TC_REQUIRE(spec, "null spec");
+    spec[0] = splits;
     workspace_elems(info, batch, capacity, kv_heads, num_splits, splits, &spec[1], &spec[2]);
-    spec[0] = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
     return TC_OK;
 }
 
@@ -1416,9 +1410,8 @@ int tc_decode_resources(int device, int64_t batch, int64_t capacity, int64_t kv_
     const int64_t slots = plan_slots(info, batch, capacity, kv_heads, num_splits);
     int64_t o_elems, lse_elems;
     workspace_elems(info, batch, capacity, kv_heads, num_splits, splits, &o_elems, &lse_elems);
-    splits = workspace_splits(info, batch, capacity, kv_heads, num_splits, splits);
     const int64_t header[12] = {splits, kGroup, kv_heads, kGroup, 1, slots > 0 ? slots * kv_heads : batch * kv_heads * splits,
-                                splits > 1 ? batch * kv_heads : 0, o_elems, lse_elems, kGroup, kTileN, 1};
+                                o_elems > 0 ? batch * kv_heads : 0, o_elems, lse_elems, kGroup, kTileN, 1};
     for (int i = 0; i < 12; ++i) values[i] = header[i];
     status = mapping == 1 ? tc::kernel_resources(&decode_splitkv_kernel<true, false>, kThreads, shared_bytes(true), values + 12)
                           : tc::kernel_resources(&decode_splitkv_kernel<false, false>, kThreads, shared_bytes(false), values + 12);
