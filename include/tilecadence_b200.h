@@ -242,8 +242,8 @@ int tc_decode_rope_forward_out(int device, void* stream, const void* q, void* kc
  * (peer_blocks[rank] is this rank's own block). All ranks must make the same sequence of calls with
  * the same batch, kv_heads and world on the same blocks. peer_block_size is the size in bytes every one of
  * those blocks was created with; a call whose (batch, kv_heads, world) needs more than that is rejected,
- * because its stores would leave the blocks on the other GPUs. splits * Hkv * B CTAs must be resident at
- * once (rejected otherwise). Plain stores only; no collective library call is involved.
+ * because its stores would leave the blocks on the other GPUs. All CTAs of the launch (splits * Hkv * B, or what a
+ * split by length takes, at most two to an SM) must be resident at once (rejected otherwise). Plain stores only; no collective library call is involved.
  *
  * Exchange blocks: tc_peer_block_bytes gives the size for (batch, kv_heads, world);
  * tc_peer_block_create allocates and zeroes one on `device` and returns a 64-byte interprocess handle;

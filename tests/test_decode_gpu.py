@@ -624,3 +624,37 @@ def test_the_workspace_spec_still_names_the_split_count(gpu_device, batch, capac
                         *(torch.full((n,), float("nan"), device=gpu_device) for n in workspace[1:]), num_splits, 1, True)
         results.append((out.cpu(), lse.cpu()))
     assert torch.equal(bits(results[0][0]), bits(results[1][0])) and torch.equal(results[0][1], results[1][1])
+
+
+def test_exchange_grid_is_checked_against_what_the_gpu_holds(gpu_device, tmp_path):
+    """A CTA of the exchange launch waits for other ranks, so its grid is refused unless the GPU holds all of it at once.
+    A build with a five-stage ring has room for one CTA to an SM, not for the two that its configuration names: 148
+    CTAs are taken and give the plain result, twice as many are refused (a world of one: nobody waits here)."""
+    from tilecadence_b200 import operator, sharding
+
+    operator.emit("decode", tmp_path / "decode")
+    path, _ = cuda_runtime.compile_directory(tmp_path / "decode", defines=("AB_DECODE_STAGES=5",))
+    ops = cuda_runtime.ops_for(cuda_runtime.load_library(path), "decode")
+    sms = torch.cuda.get_device_properties(gpu_device).multi_processor_count
+    q, kcache, vcache, knew, vnew = make_case(41, 1, 4096)
+    old = torch.tensor([4000], dtype=torch.int32)
+    fits = sms // 8
+    want_o, _, want_k, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, num_splits=fits)
+    dq, dk, dv, dkn, dvn, dold = (t.to(gpu_device) for t in (q, kcache, vcache, knew, vnew, old))
+    resources = ops.resources(dq, dk, dold, 0, 1, True)
+    assert resources[19] == 1
+    for splits in (fits, 2 * fits):
+        driver = sharding.ShardedDecode(ops, 0, 1, 1, 4096, gpu_device, exchange="peer")
+        out, lse = torch.empty_like(dq), torch.empty((1, 32, 1), device=gpu_device)
+        try:
+            if splits == fits:
+                driver.step(dq, dk, dv, dkn, dvn, dold, out, lse, num_splits=splits)
+                torch.cuda.synchronize()
+                assert torch.equal(bits(out.cpu()), bits(want_o)) and torch.equal(bits(dk.cpu()), bits(want_k))
+            else:
+                with pytest.raises(RuntimeError, match=f"co-resident, {sms} fit"):
+                    driver.step(dq, dk, dv, dkn, dvn, dold, out, lse, num_splits=splits)
+        finally:
+            driver.close()
+    shipped = cuda_runtime.default_ops("decode").resources(dq, dk, dold, 0, 1, True)
+    assert shipped[19] == 2  # what the admission by the configuration counts on

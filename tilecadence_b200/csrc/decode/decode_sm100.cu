@@ -1018,19 +1018,32 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
     auto kernel = &decode_splitkv_kernel<kHandoff, kPeer>;
     constexpr int shared = shared_bytes(kHandoff);
     static thread_local int configured_device = -1;
+    static thread_local int64_t resident_ctas = 0;
     int device = 0;
     TC_CUDA(cudaGetDevice(&device));
     if (configured_device != device) {
         const int status = tc::raise_shared_limit(kernel, kSpreadShared);
         if (status != TC_OK) return status;
+        if (kPeer) {
+            int sms = 0, active = 0;
+            TC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+            TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, kernel, kThreads, shared));
+            resident_ctas = int64_t(sms) * active;
+        }
         configured_device = device;
     }
     cudaLaunchConfig_t config{};
     const int depth = p.plan_slots > 0 ? (p.plan_slots + p.splits - 1) / p.splits : p.batch;
+    // Every CTA of the grid must be resident at once: a CTA that waits for another rank holds its slot, and the CTAs it
+    // indirectly waits for on that rank must never queue behind waiters. What fits is asked of this very kernel.
+    if (kPeer)
+        TC_REQUIRE(int64_t(p.splits) * p.kv_heads * depth <= resident_ctas,
+                   "peer exchange needs its %lld CTAs to be co-resident, %lld fit; lower num_splits",
+                   static_cast<long long>(int64_t(p.splits) * p.kv_heads * depth), static_cast<long long>(resident_ctas));
     // One CTA per SM, by asking for more than half of its shared memory: see plan_slots, and a grid that may start before
     // its predecessor ends and then finds some SMs emptier than others (four caches of 4096 in a chain of layers: 16.1
     // -> 15.1 us).
-    // Never with peers: their CTAs wait for other ranks, so all of the grid's have to be resident at once.
+    // Never with peers, whose grid has to be resident as a whole.
     const bool spread = !kPeer && p.plan_slots > 0 && (p.splits == 1 ? p.plan_even > p.batch : p.cache_stable != 0);
     config.gridDim = dim3(p.splits, p.kv_heads, depth);
     config.blockDim = dim3(kThreads);
@@ -1121,9 +1134,7 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
         for (int r = 0; r < peer->world; ++r)
             TC_REQUIRE(peer->blocks[r] && reinterpret_cast<uintptr_t>(peer->blocks[r]) % 16 == 0,
                        "every rank's exchange block must be mapped and 16-byte aligned");
-        // Every CTA of the grid must be resident at once: a CTA that waits for another rank holds
-        // its slot, and the CTAs it indirectly waits for on that rank must never queue behind waiters.
-        // (A launch that splits by length never has more CTAs than fit.)
+        // (checked again at the launch, against what this GPU holds of the kernel)
         TC_REQUIRE(int64_t(splits) * kv_heads * batch <= int64_t(info.sms) * AB_DECODE_CTAS_PER_SM,
                    "peer exchange needs splits*Hkv*B CTAs to be co-resident; lower num_splits");
     }
