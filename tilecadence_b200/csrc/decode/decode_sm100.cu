@@ -482,7 +482,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             return true;
         };
         if (!p.block_table) {
-            // (lane 0, not an elected lane: 11.2 against 11.5 us for one sequence of 8192 rows under the promise)
+            // (lane 0, not an elected lane: 10.7 against 11.2 us for one sequence of 8192 rows under the promise)
             if (lane == 0) {
                 const int ring_early = early_tiles < kStages ? early_tiles : kStages;
                 bool ok = true;
@@ -972,8 +972,7 @@ int auto_splits(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int
 // * where even splits are two or more: as many as those, so that equal lengths leave no CTA idle (with idle CTAs in the
 //   grid, launches that overlap their predecessor's end settle two CTAs on one SM and none on another: 90 us against
 //   81 at four full caches of 32768);
-// * else as many as fill both CTA slots of every SM. Up to one sequence per SM they are kept one to an SM all the
-//   same, for the same reason (16 equal sequences of 2000: 25.9 us, kept apart 23.6, even splits 22.9).
+// * else as many as fill both CTA slots of every SM.
 // Where even splits leave no share longer than a merge costs there is nothing to gain.
 constexpr int kPlanMaxBatch = 64;  // two sequences per lane
 int plan_even(const tc::DeviceInfo& info, int64_t batch, int64_t kv_heads) {
@@ -986,6 +985,23 @@ int plan_slots(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int6
     const int64_t splits = auto_splits(info, batch, capacity, kv_heads), tiles = (capacity + kTileN - 1) / kTileN;
     if (tiles <= splits * int64_t(kMergeCost)) return 0;
     return int(splits > 1 ? splits * batch : both);
+}
+// Whether a launch with `slots` slots keeps its CTAs one to an SM, by asking for more than half of the shared memory (us,
+// kept apart against two to an SM):
+// * One split each: while fewer sequences than one to an SM leave SMs free. 12 / 16 equal ones of 2000 rows 21.5 / 23.3
+//   against 23.2 / 24.0. (Unequal ones would rather share: 16 of 500-8000 rows 42.4 against 37.8. At exactly one to an SM,
+//   18, equal ones take 25.6 against 26.2 and unequal ones 37.3 against 31.3: not kept apart.)
+// * Two or more splits, under a promise: the launch may start before its predecessor ends and would find some SMs emptier
+//   than others. Behind another kernel than a decode step that is worth more than the early start beside its CTAs, at any
+//   length: a layer of four caches of 4096 rows 23.4 against 25.4, of eight 32.1 against 36.3 (even where a decode CTA and
+//   the projection's fit one SM together). Behind a decode step of the same caches it pays while shares use the promise:
+//   four caches of 4096 13.9 against 15.5, but of 8192 24.9 against 23.9 and eight of 8192 44.9 against 43.5.
+bool one_per_sm(const tc::DeviceInfo& info, int64_t slots, int splits, int64_t batch, int64_t capacity, int64_t kv_heads,
+                int cache_stable) {
+    if (slots == 0) return false;
+    if (splits == 1) return batch < info.sms / kv_heads;
+    const int64_t tiles = (capacity + kTileN - 1) / kTileN;
+    return cache_stable == 1 || (cache_stable == 2 && tiles <= int64_t(splits) * kEarlyLimitTiles);
 }
 // FP32 elements of the workspace that a launch with `slots` slots uses: the partial O and LSE of every slot, behind
 // the LSEs one 8-byte ticket per (batch, KV head).
@@ -1018,7 +1034,7 @@ int check_geometry(int device, int64_t batch, int64_t capacity, int64_t kv_heads
 }
 
 template <bool kHandoff, bool kPeer, bool kByLength>
-int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, cudaStream_t stream) {
+int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, bool spread, cudaStream_t stream) {
     auto kernel = &decode_splitkv_kernel<kHandoff, kPeer, kByLength>;
     constexpr int shared = shared_bytes(kHandoff);
     static thread_local int configured_device = -1;
@@ -1044,11 +1060,6 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
         TC_REQUIRE(int64_t(p.splits) * p.kv_heads * depth <= resident_ctas,
                    "peer exchange needs its %lld CTAs to be co-resident, %lld fit; lower num_splits",
                    static_cast<long long>(int64_t(p.splits) * p.kv_heads * depth), static_cast<long long>(resident_ctas));
-    // One CTA per SM, by asking for more than half of its shared memory: see plan_slots, and a grid that may start before
-    // its predecessor ends and then finds some SMs emptier than others (four caches of 4096 in a chain of layers: 16.1
-    // -> 15.1 us).
-    // Never with peers, whose grid has to be resident as a whole.
-    const bool spread = !kPeer && kByLength && (p.splits == 1 ? p.plan_even > p.batch : p.cache_stable != 0);
     config.gridDim = dim3(p.splits, p.kv_heads, depth);
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = spread ? kSpreadShared : shared;
@@ -1063,10 +1074,11 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
 }
 
 template <bool kPeer>
-int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, bool handoff, void* stream) {
+int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, bool handoff, bool spread, void* stream) {
     const auto s = static_cast<cudaStream_t>(stream);
-    if (p.plan_slots > 0) return handoff ? launch<true, kPeer, true>(kmap, vmap, p, s) : launch<false, kPeer, true>(kmap, vmap, p, s);
-    return handoff ? launch<true, kPeer, false>(kmap, vmap, p, s) : launch<false, kPeer, false>(kmap, vmap, p, s);
+    if (p.plan_slots > 0)
+        return handoff ? launch<true, kPeer, true>(kmap, vmap, p, spread, s) : launch<false, kPeer, true>(kmap, vmap, p, spread, s);
+    return handoff ? launch<true, kPeer, false>(kmap, vmap, p, false, s) : launch<false, kPeer, false>(kmap, vmap, p, false, s);
 }
 
 struct PeerArgs {
@@ -1253,9 +1265,10 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
         p.world = peer->world;
         p.rank = peer->rank;
         for (int r = 0; r < peer->world; ++r) p.peer_blocks[r] = static_cast<uint8_t*>(peer->blocks[r]);
-        return launch<true>(kmap, vmap, p, mapping == 1, stream);
+        return launch<true>(kmap, vmap, p, mapping == 1, false, stream);  // never spread: the whole grid has to be resident
     }
-    return launch<false>(kmap, vmap, p, mapping == 1, stream);
+    const bool spread = one_per_sm(info, slots, splits, batch, capacity, kv_heads, cache_stable);
+    return launch<false>(kmap, vmap, p, mapping == 1, spread, stream);
 }
 
 
@@ -1358,7 +1371,7 @@ int decode_static(int device, void* stream, const void* q, void* kcache, void* v
     p.cache_slots = int(batch);
     p.scale = 1.f / std::sqrt(128.f);
     p.scale_log2 = p.scale * float(M_LOG2E);
-    return launch<false>(kmap, vmap, p, mapping == 1, stream);
+    return launch<false>(kmap, vmap, p, mapping == 1, false, stream);
 }
 
 }  // namespace
@@ -1434,7 +1447,8 @@ int tc_decode_resources(int device, int64_t batch, int64_t capacity, int64_t kv_
     for (int i = 0; i < 12; ++i) values[i] = header[i];
     const auto kernel = slots > 0 ? (mapping == 1 ? &decode_splitkv_kernel<true, false, true> : &decode_splitkv_kernel<false, false, true>)
                                   : (mapping == 1 ? &decode_splitkv_kernel<true, false, false> : &decode_splitkv_kernel<false, false, false>);
-    status = tc::kernel_resources(kernel, kThreads, shared_bytes(mapping == 1), values + 12);
+    const bool spread = one_per_sm(info, slots, splits, batch, capacity, kv_heads, 0);
+    status = tc::kernel_resources(kernel, kThreads, spread ? kSpreadShared : shared_bytes(mapping == 1), values + 12);
     if (status != TC_OK) return status;
     status = tc::kernel_resources(&combine_partials_kernel, 128, 0, values + 20);
     if (status != TC_OK) return status;
