@@ -105,7 +105,7 @@ int tc_prefill_resources(int device, const int64_t q_strides[3], const int64_t k
  * given for every sequence. 0 leaves it open, and spec[0] is the count that the SM number gives every sequence. A batch
  * of 2 to 64 sequences may then be split on the device by the lengths it finds there: spec[1] and spec[2] are the
  * workspace that this takes, larger than spec[0] splits need and not zero where spec[0] == 1 (the partials and, behind
- * the LSEs, 2 elements of ticket per (sequence, KV head)); it needs no initial value. With a workspace that holds
+ * the LSEs, 4 elements of ticket per (sequence, KV head)); it needs no initial value. With a workspace that holds
  * spec[0] splits only, those are what the call uses.
  */
 int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,

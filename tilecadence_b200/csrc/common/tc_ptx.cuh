@@ -103,6 +103,13 @@ __device__ __forceinline__ bool wait_word_gpu(const int32_t* address, int32_t ex
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// 16 bytes from global (through L2) to shared memory, both 16-byte aligned; the issuing thread may read them there after
+// copies_wait().
+__device__ __forceinline__ void copy_16_async(void* shared, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(shared)), "l"(global) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ int atomic_add_acq_rel(int* address, int value) {
     int old;
     asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(address), "r"(value) : "memory");

@@ -62,7 +62,7 @@ constexpr int kMaxSplits = 128;
 constexpr int kPrefetchTiles = 12;  // tiles a CTA may prefetch into L2 beyond its shared-memory ring
 constexpr int kEarlyLimitTiles = 32;  // shares longer than this stream nothing ahead of the stream dependency
 // A launch that splits by length counts its finished shares in the caller's workspace, which holds anything at first:
-// a ticket word is this pattern plus the count, and whoever finds another value arms it (see arm_ticket). The pattern's
+// a ticket word is this pattern plus the count, and whoever finds another value arms it (see take_ticket). The pattern's
 // upper half is a NaN with a payload, which no partial result left there by another launch has.
 constexpr unsigned long long kArmed = 0xffa5c3d296e17b00ull;
 constexpr int kStagingBytes = 2304;  // dedicated O/LSE staging when the handoff is disabled
@@ -85,6 +85,7 @@ __host__ __device__ constexpr size_t peer_block_bytes(int world, int units) {
     return (peer_epochs_offset(world, units) + size_t(units) * 4 + 255) / 256 * 256;
 }
 
+static_assert((kGroups * kStages + kStages) * 8 + 4 <= kBarrierBytes - 16, "barriers, the flag and a copy of the ticket");
 static_assert(kStageBytes == 2 * kVBytes, "a stage holds one V tile followed by one K tile");
 static_assert(kMaxSplits % 32 == 0 && kGroup * kMaxSplits * 4 <= kVBytes, "split weights fit the terminal K stage");
 static_assert(kTileN == 16 * kGroupWarps, "each warp of a consumer group owns 16 keys of a tile");
@@ -118,7 +119,7 @@ struct DecodeParams {
     float* ws_o;
     float* ws_lse;
     int32_t* tickets;
-    unsigned long long* plan_tickets;  // splits by length: [B * Hkv] in the workspace
+    ulonglong2* plan_tickets;  // splits by length: [B * Hkv] in the workspace, the count in the first word
     int32_t* status;
     int batch, capacity, kv_heads, splits, append, partial;
     // Splits by length (0: every sequence gets `splits`): the grid holds plan_slots CTAs per KV head, dealt to the
@@ -273,13 +274,14 @@ __device__ __forceinline__ Share plan_share(const DecodeParams& p, int slot, int
     return share;
 }
 
-// Every CTA of a split sequence arms the ticket of its (batch, KV head) once the preceding kernel has completed and
-// long before it takes the ticket: the first one to get there sets the count to zero, the others find the pattern (or
-// lose the exchange to one that does). The last CTA leaves the word armed for the next launch. The words belong to the
-// call's own workspace, so calls on different streams with buffers of their own do not meet here.
-__device__ __forceinline__ void arm_ticket(unsigned long long* ticket) {
-    const unsigned long long found = __ldcg(ticket);
-    if ((found & ~0xffull) != kArmed) atomicCAS(ticket, found, kArmed);
+// Ticket of a launch split by length, for one thread of each CTA. Whoever found the word unarmed tries to arm it with a
+// count of zero (one exchange succeeds; the others find it armed, or armed and counted) before it counts itself. `found`
+// was read any time since the preceding kernel completed: a word once armed stays so. The last CTA leaves the word
+// armed for the next launch. The words belong to the call's own workspace, so calls on different streams with buffers of
+// their own do not meet here.
+__device__ __forceinline__ bool take_ticket(ulonglong2* ticket, unsigned long long found, int splits) {
+    if ((found & ~0xffull) != kArmed) atomicCAS(&ticket->x, found, kArmed);
+    return tc::atomic_add_acq_rel(&ticket->x, 1ull) == kArmed + uint32_t(splits - 1);
 }
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory"); }
@@ -361,6 +363,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);  // [kGroups][kStages]
     uint64_t* empty = full + kGroups * kStages;
     int* flag = reinterpret_cast<int*>(empty + kStages);
+    ulonglong2* ticket_seen = reinterpret_cast<ulonglong2*>(smem + kStages * kStageBytes + kBarrierBytes - sizeof(ulonglong2));
     uint8_t* staging = kHandoff ? smem : smem + kStages * kStageBytes + kBarrierBytes;
     float* stage_o = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_O_OFFSET_BYTES : 0));
     float* stage_lse = reinterpret_cast<float*>(staging + (kHandoff ? AB_DECODE_LSE_OFFSET_BYTES : 2048));
@@ -530,6 +533,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     }
 
     // ---------------------------------------------------------------------- consumer warps
+    // The ticket word travels beside the work (read in the epilogue it cost 0.4 us; read into a register here, 0.3 where
+    // the tiles are early).
+    if (kByLength && splits > 1 && threadIdx.x == 0)
+        tc::copy_16_async(ticket_seen, p.plan_tickets + int64_t(b) * p.kv_heads + kvh);
     const int qrow = lane >> 2;       // query head within the group; rows >= 4 are padding
     const int quad = lane & 3;
     const bool row_ok = qrow < kGroup;
@@ -573,7 +580,6 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     // Tile `it` belongs to group (n_tiles - 1 - it) % kGroups: the last tile, which lands in stage 0, to group 0,
     // the one before it (stage 1) to group 1. A group's last tile therefore sits in the stage of its own number.
     const int group = warp / kGroupWarps, gw = warp % kGroupWarps;
-    if (kByLength && splits > 1 && threadIdx.x == 0) arm_ticket(p.plan_tickets + int64_t(b) * p.kv_heads + kvh);
     const int first_tile = (((n_tiles - 1 - group) % kGroups) + kGroups) % kGroups;
 
     for (int it = first_tile; it < n_tiles; it += kGroups) {
@@ -780,9 +786,14 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         // The barrier orders every thread's partial stores before thread 0's release; the last
         // arriver's acquire, followed by the second barrier, orders them before the merge loads.
         merge_barrier();
-        if (tid == 0)
-            *flag = kByLength ? tc::atomic_add_acq_rel(p.plan_tickets + head_slot, 1ull) == kArmed + uint32_t(splits - 1)
-                              : tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
+        if (tid == 0) {
+            if constexpr (kByLength) {
+                tc::copies_wait();
+                *flag = take_ticket(p.plan_tickets + head_slot, ticket_seen->x, splits);
+            } else {
+                *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
+            }
+        }
         merge_barrier();
         TC_TRACE_POINT(22);
         if (!*flag) return;
@@ -849,7 +860,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         // Every split of this head has taken its ticket: a plain store re-arms the counter for the next launch
         // (an atomic exchange would keep this CTA, and with it the end of the kernel, waiting for its return).
         if (tid == 0) {
-            if (kByLength) p.plan_tickets[head_slot] = kArmed;
+            if (kByLength) p.plan_tickets[head_slot].x = kArmed;
             else p.tickets[head_slot] = 0;
         }
     } else {
@@ -1004,9 +1015,11 @@ bool one_per_sm(const tc::DeviceInfo& info, int64_t slots, int splits, int64_t b
     return cache_stable == 1 || (cache_stable == 2 && tiles <= int64_t(splits) * kEarlyLimitTiles);
 }
 // FP32 elements of the workspace that a launch with `slots` slots uses: the partial O and LSE of every slot, behind
-// the LSEs one 8-byte ticket per (batch, KV head).
+// the LSEs one 16-byte ticket per (batch, KV head).
 int64_t plan_o_elems(int64_t slots, int64_t kv_heads) { return slots * kv_heads * kGroup * kDim; }
-int64_t plan_lse_elems(int64_t slots, int64_t batch, int64_t kv_heads) { return slots * kv_heads * kGroup + (slots > 0 ? batch * kv_heads * 2 : 0); }
+int64_t plan_lse_elems(int64_t slots, int64_t batch, int64_t kv_heads) {
+    return slots * kv_heads * kGroup + (slots > 0 ? batch * kv_heads * int64_t(sizeof(ulonglong2) / 4) : 0);
+}
 // What tc_decode_workspace_spec and tc_decode_resources report: room for either kind of launch.
 void workspace_elems(const tc::DeviceInfo& info, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                      int splits, int64_t* o_elems, int64_t* lse_elems) {
@@ -1248,7 +1261,7 @@ int decode_common(int device, void* stream, const void* q, void* kcache, void* v
     p.ws_o = workspace_o;
     p.ws_lse = workspace_lse;
     p.tickets = scratch.tickets;
-    if (slots > 0) p.plan_tickets = reinterpret_cast<unsigned long long*>(workspace_lse + int64_t(slots) * kv_heads * kGroup);
+    if (slots > 0) p.plan_tickets = reinterpret_cast<ulonglong2*>(workspace_lse + int64_t(slots) * kv_heads * kGroup);
     p.status = scratch.status;
     p.batch = int(batch);
     p.capacity = int(capacity);
