@@ -658,3 +658,23 @@ def test_exchange_grid_is_checked_against_what_the_gpu_holds(gpu_device, tmp_pat
             driver.close()
     shipped = cuda_runtime.default_ops("decode").resources(dq, dk, dold, 0, 1, True)
     assert shipped[19] == 2  # what the admission by the configuration counts on
+
+
+@pytest.mark.parametrize("batch,capacity,apart", [(4, 4096, 512), (4, 4096, 513), (16, 2048, 128), (16, 2048, 129), (33, 2048, 128),
+                                                  (33, 2048, 129)])
+def test_close_lengths_are_split_evenly(gpu_device, batch, capacity, apart):
+    """Lengths within two tiles per even split of each other (the last one shortest, the middle one longest) take the
+    places of even splits, the next row makes the launch plan; either way the result agrees with one split each, and
+    close lengths give the bits of the launch with that split count."""
+    ops = cuda_runtime.default_ops("decode")
+    lengths = [capacity - 100 - (b * 7) % (apart // 2) for b in range(batch)]
+    lengths[batch // 2], lengths[-1] = capacity - 100, capacity - 100 - apart
+    q, kcache, vcache, knew, vnew = make_case(7, batch, capacity, fill=lengths)
+    old = torch.tensor(lengths, dtype=torch.int32)
+    one_o, one_lse, one_k, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, num_splits=1)
+    got_o, got_lse, got_k, _, spec = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old)
+    oracle.check_outputs(got_o, got_lse, one_o.float(), one_lse)
+    assert torch.equal(bits(got_k), bits(one_k))
+    even_o, even_lse, _, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, num_splits=spec[0])
+    if apart == 128 * spec[0]:
+        assert torch.equal(bits(got_o), bits(even_o)) and torch.equal(got_lse, even_lse)

@@ -180,14 +180,16 @@ __device__ __forceinline__ int64_t old_length(const DecodeParams& p, int b) {
     const int64_t length = p.old_lengths[b];
     return length < 0 ? 0 : length;
 }
-__device__ __forceinline__ int visible_rows(const DecodeParams& p, int64_t old_len) {
+template <class Params>
+__device__ __forceinline__ int visible_rows(const Params& p, int64_t old_len) {
     const int64_t visible = old_len + (p.append ? 1 : 0) - p.shard_start;
     return int(visible < 0 ? 0 : (visible > p.capacity ? p.capacity : visible));
 }
 
-// Which share of which sequence a CTA of a launch that splits by length works on: sequence b is cut into
-// ceil(tiles_b / size) even shares, at least one. One warp of each CTA works it out from the lengths on the device,
-// every one with the same answer.
+// Which share of which sequence a CTA of a launch that splits by length works on. Lengths so close that the shares of even
+// splits differ by two tiles at most are split evenly, by the CTA's place in the grid. Others come here: sequence b is
+// cut into ceil(tiles_b / size) even shares, at least one. One warp of each CTA works it out from the lengths on the
+// device, every one with the same answer.
 //
 // Why: with the same number of splits for every sequence the longest one sets the time of a ragged batch (one CTA
 // takes a 32 KiB tile in about 0.56 us alone, whatever the others do), while the stream as a whole needs about 112
@@ -195,32 +197,35 @@ __device__ __forceinline__ int visible_rows(const DecodeParams& p, int64_t old_l
 //   max(longest share, all tiles / 112), and what the shares cost on top:
 //   kMergeCost if any sequence is split (partials, tickets, the last CTA's merge), and if there are more shares
 //   than put one CTA on every SM, kSecondCost and a twelfth of the stream.
-// Equal lengths, and lengths of which none outlasts the stream by what a split costs, need no search: the even split
-// count, or one. Measured (us, even splits before, by length now): 16 paged sequences of 500-8000 rows 72.7 -> 43.5, 24
-// of 300-5000 52.7 -> 33.7, 8 of 200-3333 20.2 -> 15.1; equal lengths pay 0.1 to 0.8 for the look at all of them.
+// Lengths of which none outlasts the stream by what a split costs need no search: they are not split.
+// Measured (us, even splits before, by length now): 16 sequences of 500-8000 rows 70.3 -> 41.9, 24 of 300-5000
+// 52.9 -> 33.9, 8 of 200-3333 20.0 -> 14.8. Equal lengths pay for the look at all of them: 8 of 2000 rows 15.3 -> 15.5,
+// 2 of 8192 15.6 -> 15.9; a search, where lengths are close, cost 0.9 at four of about 2000 (11.9 against 11.0).
+// Out of line: inlined ahead of the first load it cost every launch 0.1 to 0.2.
 struct Share {
     int b, split, splits, first;  // first: slot of the sequence's first share; splits == 0: nothing to do
     int old_length;
 };
 constexpr float kStreamCtas = 112, kMergeCost = 8, kSecondCost = 2;
-__device__ __forceinline__ Share plan_share(const DecodeParams& p, int slot, int lane) {
+struct PlanInput {
+    int64_t shard_start;
+    int batch, capacity, kv_heads, append, plan_slots, plan_even;
+};
+// length0, length1: of this lane's sequences, `lane` and `lane + 32`; lanes beyond the batch repeat its last one (for the
+// extremes) with a weight of 0 (for the sums).
+__device__ __noinline__ void plan_share(const PlanInput p, int length0, int length1, int slot, int lane, Share* out) {
     constexpr uint32_t kAll = 0xffffffffu;
     const int last = p.batch - 1;
-    // Lanes beyond the batch repeat its last sequence (for the extremes) with a weight of 0 (for the sums).
-    const int64_t old0 = old_length(p, lane < last ? lane : last), old1 = old_length(p, lane + 32 < last ? lane + 32 : last);
+    const int old0 = max(length0, 0), old1 = max(length1, 0);
     const uint32_t t0 = uint32_t(visible_rows(p, old0) + kTileN - 1) / kTileN, t1 = uint32_t(visible_rows(p, old1) + kTileN - 1) / kTileN;
     const bool two = p.batch > 32;
     const uint32_t total = __reduce_add_sync(kAll, (lane <= last ? t0 : 0u) + (lane + 32 <= last ? t1 : 0u));
     const uint32_t longest = __reduce_max_sync(kAll, two && t1 > t0 ? t1 : t0);
-    const uint32_t shortest = __reduce_min_sync(kAll, two && t1 < t0 ? t1 : t0);
     const float stream = float(total) * float(p.kv_heads) * (1.f / kStreamCtas);
     Share share{};
-    if (longest == shortest || float(longest) <= stream + kMergeCost + kSecondCost) {
-        share.splits = longest == shortest ? p.splits : 1;
-        share.b = share.splits == 1 ? slot : slot / share.splits;
-        share.first = share.b * share.splits;
-        share.split = slot - share.first;
-        if (share.b > last) share.splits = 0;
+    if (float(longest) <= stream + kMergeCost + kSecondCost) {
+        share.splits = slot <= last;
+        share.b = share.first = slot <= last ? slot : 0;
     } else {
         // ceil(tiles / size), at least 1, as a float and without a division or a conversion: adding 2^23 rounds up to
         // a whole number. Beyond 2^21 tiles it may be off by one, the same in every thread.
@@ -268,10 +273,9 @@ __device__ __forceinline__ Share plan_share(const DecodeParams& p, int slot, int
             share.first += __shfl_sync(kAll, end, 31);
         }
     }
-    // (int32 on the device, so the length fits again)
-    const int length0 = __shfl_sync(kAll, int(old0), share.b & 31), length1 = __shfl_sync(kAll, int(old1), share.b & 31);
-    share.old_length = share.b < 32 ? length0 : length1;
-    return share;
+    const int found0 = __shfl_sync(kAll, old0, share.b & 31), found1 = __shfl_sync(kAll, old1, share.b & 31);
+    share.old_length = share.b < 32 ? found0 : found1;
+    if (lane == 0) *out = share;
 }
 
 // Ticket of a launch split by length, for one thread of each CTA. Whoever found the word unarmed tries to arm it with a
@@ -401,19 +405,39 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
 
     // Device-side lengths: no host read.
     Share share{int(blockIdx.z), int(blockIdx.x), p.splits, 0, 0};
+    __shared__ Share planned;  // split by length: the CTA's share, as the producer warp saw it
     if constexpr (kByLength) {
-        __shared__ Share planned;
+        // Every warp looks at all lengths and knows without waiting for another whether they are close; if so its share
+        // is its place in the grid (every CTA decides alike). If not, the producer warp plans for the CTA. Which warps
+        // leave and which meet at the barriers of the epilogue follows from `planned` alone: a broken promise may show
+        // the warps different lengths, and none must wait for a warp that has left (waits for tiles end by themselves).
+        // (All warps taking the producer's answer instead: 0.2 to 0.4 us more; a barrier that also votes: 0.6.)
+        const int last = p.batch - 1;
+        share.b = share.b < last ? share.b : last;
+        share.old_length = p.old_lengths[share.b];
+        // (lanes beyond the batch repeat its last sequence)
+        const int32_t old0 = p.old_lengths[lane < last ? lane : last];
+        const int32_t old1 = p.batch > 32 ? p.old_lengths[lane + 32 < last ? lane + 32 : last] : old0;
+        const uint32_t apart = uint32_t(__reduce_max_sync(0xffffffffu, max(old0, old1))) -
+                               uint32_t(__reduce_min_sync(0xffffffffu, min(old0, old1)));
+        const bool close = apart <= uint32_t(2 * kTileN * p.splits);
+        share.old_length = max(share.old_length, 0);
+        share.first = share.b * p.splits;
+        if (int(blockIdx.z) > last) share.splits = 0;
         if (warp == kConsumerWarps) {
-            const Share mine = plan_share(p, int(blockIdx.x + blockIdx.z * gridDim.x), lane);
-            if (lane == 0) planned = mine;
+            if (!close)
+                plan_share({p.shard_start, p.batch, p.capacity, p.kv_heads, p.append, p.plan_slots, p.plan_even}, old0, old1,
+                           int(blockIdx.x + blockIdx.z * gridDim.x), lane, &planned);
+            else if (lane == 0)
+                planned = share;
         }
         __syncthreads();
-        share = planned;
-        if (share.splits == 0) return;  // more slots than shares
+        if (!close) share = planned;
+        if (share.splits == 0 && planned.splits == 0) return;  // more slots than shares
     }
-    const int b = share.b, split = share.split, splits = share.splits;
-    const int64_t old_len = kByLength ? share.old_length : old_length(p, b);
-    const int n_valid = visible_rows(p, old_len);
+    const int64_t old_len = kByLength ? share.old_length : old_length(p, share.b);
+    const int b = share.b, split = share.split, splits = kByLength ? max(share.splits, 1) : share.splits;
+    const int n_valid = kByLength && share.splits == 0 ? 0 : visible_rows(p, old_len);
     const int64_t append_local = old_len - p.shard_start;
     const bool do_append = p.append && append_local >= 0 && append_local < p.capacity;
     const int append_row = do_append ? int(append_local) : -1;
@@ -721,6 +745,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     // Quad-partial row sums become full sums; each warp parks its partial in the K rows it owns in its
     // group's terminal stage (nobody else reads those rows: the group is done with them and the other
     // group never reads that stage again), then one barrier releases the stages.
+    if constexpr (kByLength) {
+        share = planned;  // read again here: held in registers over the key loop it cost more
+        if (share.splits == 0) return;
+    }
     row_sum += __shfl_xor_sync(0xffffffffu, row_sum, 1);
     row_sum += __shfl_xor_sync(0xffffffffu, row_sum, 2);
     uint8_t* terminal_k = smem + kVBytes;  // K tile of stage 0; group g parks in the K tile of stage g
@@ -771,15 +799,15 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     merge_barrier();  // publish the four output rows and their LSE together
     TC_TRACE_POINT(21);
 
-    const int64_t head_slot = int64_t(b) * p.kv_heads + kvh;  // index of the (batch, KV head) pair
+    const int64_t head_slot = int64_t(share.b) * p.kv_heads + kvh;  // index of the (batch, KV head) pair
     float4 final_o;
     float final_lse;
-    if (splits > 1) {
+    if (share.splits > 1) {
         // Partials of a (batch, KV head) pair are `slot_step` slots apart.
         const int64_t first_slot = kByLength ? int64_t(share.first) * p.kv_heads + kvh : head_slot;
         const int64_t slot_step = kByLength ? p.kv_heads : int64_t(p.batch) * p.kv_heads;
         // Vector export of the staged tile: one 16-byte word per thread.
-        const int64_t slot = split * slot_step + first_slot;
+        const int64_t slot = share.split * slot_step + first_slot;
         reinterpret_cast<uint4*>(p.ws_o + slot * (kGroup * kDim))[tid] = reinterpret_cast<const uint4*>(stage_o)[tid];
         if (tid == 0)
             *reinterpret_cast<uint4*>(p.ws_lse + slot * kGroup) = *reinterpret_cast<const uint4*>(stage_lse);
@@ -789,9 +817,9 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         if (tid == 0) {
             if constexpr (kByLength) {
                 tc::copies_wait();
-                *flag = take_ticket(p.plan_tickets + head_slot, ticket_seen->x, splits);
+                *flag = take_ticket(p.plan_tickets + head_slot, ticket_seen->x, share.splits);
             } else {
-                *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == splits - 1;
+                *flag = tc::atomic_add_acq_rel(p.tickets + head_slot, 1) == share.splits - 1;
             }
         }
         merge_barrier();
@@ -813,11 +841,11 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
 #pragma unroll
         for (int i = 0; i < kMaxSplits / 32; ++i) {
             const int s = col4 + 32 * i;
-            part_lse[i] = s < splits ? __ldcg(lse_base + s * stride_lse) : -INFINITY;
+            part_lse[i] = s < share.splits ? __ldcg(lse_base + s * stride_lse) : -INFINITY;
         }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)  // first batch goes out with the LSE loads: one L2 round trip
-            if (u < splits) v[u] = __ldcg(o_base + u * stride_o4);
+            if (u < share.splits) v[u] = __ldcg(o_base + u * stride_o4);
         float lse_max = -INFINITY;
 #pragma unroll
         for (int i = 0; i < kMaxSplits / 32; ++i) lse_max = fmaxf(lse_max, part_lse[i]);
@@ -836,15 +864,15 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
         __syncwarp();
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s0 = 0; s0 < splits; s0 += kBatch) {
+        for (int s0 = 0; s0 < share.splits; s0 += kBatch) {
             if (s0 > 0) {
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u)
-                    if (s0 + u < splits) v[u] = __ldcg(o_base + (s0 + u) * stride_o4);
+                    if (s0 + u < share.splits) v[u] = __ldcg(o_base + (s0 + u) * stride_o4);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const float w = s0 + u < splits ? weights[s0 + u] : 0.f;
+                const float w = s0 + u < share.splits ? weights[s0 + u] : 0.f;
                 if (w > 0.f) {  // a split that saw no key may hold anything: never multiply it
                     acc.x = fmaf(w, v[u].x, acc.x);
                     acc.y = fmaf(w, v[u].y, acc.y);
@@ -868,7 +896,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         final_lse = stage_lse[row];
     }
 
-    const int64_t out_row = int64_t(b) * q_heads + kvh * kGroup + row;
+    const int64_t out_row = int64_t(share.b) * q_heads + kvh * kGroup + row;
     if (kPeer) {
         // Cross-GPU merge inside the same launch. This CTA holds this rank's partial for the
         // (batch, KV head) unit. Every thread stores its 16 bytes of the partial, each 4-byte value
