@@ -545,9 +545,10 @@ def test_splits_by_length(gpu_device, kv_heads, lengths):
 
 
 def test_exchange_launch_split_by_length_keeps_its_grid_resident(gpu_device):
-    """Twelve sequences, more CTAs than SMs: the launch whose CTAs may wait for other ranks gives the bits of the plain
-    one, which keeps its CTAs one to an SM (asking for more shared memory, also after a look at the resources). With a
-    world of one nobody waits; the host refuses what cannot be resident."""
+    """Twelve sequences, more CTAs in the grid than SMs: the exchange launch gives the bits of the plain one, which keeps
+    its CTAs one to an SM (asking for more shared memory, also after a look at the resources). With a world of one nobody
+    waits; that the grid of an exchange launch fits is what test_exchange_grid_is_checked_against_what_the_gpu_holds is
+    about."""
     from tilecadence_b200 import sharding
 
     ops, batch, capacity = cuda_runtime.default_ops("decode"), 12, 1024
@@ -678,3 +679,53 @@ def test_close_lengths_are_split_evenly(gpu_device, batch, capacity, apart):
     even_o, even_lse, _, _, _ = run_step(ops, gpu_device, q, kcache, vcache, knew, vnew, old, num_splits=spec[0])
     if apart == 128 * spec[0]:
         assert torch.equal(bits(got_o), bits(even_o)) and torch.equal(got_lse, even_lse)
+
+
+RAGGED = {4: [3700, 250, 1200, 2500], 12: [1900, 37, 410, 65, 1700, 3, 333, 700, 128, 11, 512, 64]}
+
+
+def promised_chain(ops, device, promise, lengths, capacity, steps, caches):
+    """`steps` decode steps on one stream, every one with a length tensor of its own (rows appended one after another
+    when there is one cache, the same rows on each of several caches); outputs, LSE and caches afterwards."""
+    batch = len(lengths)
+    q, = (t.to(device) for t in oracle.seeded_normal(62, (steps, batch, 1, 32, 128)))
+    knew, vnew = (t.to(device) for t in oracle.seeded_normal(63, (steps, batch, 1, 8, 128), (steps, batch, 1, 8, 128)))
+    held = [tuple(t.to(device) for t in pair) for pair in caches]
+    olds = [torch.tensor([n + t // len(held) - (3 * b if t % 2 and len(held) > 1 else 0) for b, n in enumerate(lengths)],
+                         dtype=torch.int32, device=device).clamp_(min=0) for t in range(steps)]
+    outs = torch.full((steps, batch, 1, 32, 128), float("nan"), device=device, dtype=torch.bfloat16)
+    lses = torch.full((steps, batch, 32, 1), float("nan"), device=device)
+    spec = ops.workspace_spec(q[0], held[0][0], olds[0], 0, 1, True)
+    even = ops.workspace_spec(q[0], held[0][0], olds[0], spec[0], 1, True)
+    assert spec[1:] != even[1:]  # these calls are split by length
+    ws = [torch.full((n,), float("nan"), device=device) for n in spec[1:3]]
+    torch.cuda.synchronize()
+    for t in range(steps):
+        ops.forward_out(q[t], *held[t % len(held)], knew[t], vnew[t], olds[t], outs[t], lses[t], *ws, 0, 1, True,
+                        cache_stable=promise)
+    torch.cuda.synchronize()
+    assert ops.library.device_status(device.index) == 0
+    last = (q[-1], *held[(steps - 1) % len(held)], knew[-1], vnew[-1], olds[-1])
+    return [outs.cpu(), lses.cpu(), *(t.cpu() for pair in held for t in pair)], [t.cpu() for t in last]
+
+
+@pytest.mark.parametrize("batch,capacity", [(4, 4096), (12, 2048)])
+@pytest.mark.parametrize("promise,caches", [("prefix", 1), (True, 3)])
+def test_steps_split_by_length_may_overlap_under_a_promise(ops, gpu_device, batch, capacity, promise, caches):
+    """Ragged batches with two or more even splits and with one (whose launches have idle CTAs), steps of the same cache
+    under the prefix promise and of different caches under the cache-stable one: the lengths are read and the plan is
+    made before the step before has ended, and everything equals the chain without a promise, bit for bit."""
+    prefix = [oracle.seeded_normal(64 + c, (batch, capacity, 8, 128), (batch, capacity, 8, 128)) for c in range(caches)]
+    plain, _ = promised_chain(ops, gpu_device, False, RAGGED[batch], capacity, 12, prefix)
+    early, last = promised_chain(ops, gpu_device, promise, RAGGED[batch], capacity, 12, prefix)
+    assert not torch.isnan(plain[0].float()).any()
+    for a, b in zip(plain, early):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    q, kcache, vcache, knew, vnew, old = last  # the caches hold the last step's rows already: appended again, the same
+    want_o, want_lse, _, _ = oracle.decode_step(q, kcache, vcache, knew, vnew, old)
+    oracle.check_outputs(early[0][-1], early[1][-1], want_o, want_lse)
+
+
+def test_rotary_embedding_in_a_launch_split_by_length(ops, gpu_device):
+    lengths = [4095, 200, 3000, 64, 0, 1500, 777, 2048]
+    test_rotary_embedding_inside_the_launch(ops, gpu_device, 8, 4096, lengths, 0)

@@ -1,4 +1,4 @@
-"""The operators' native call path takes exactly the calls that the Python checks take, with the same result."""
+"""The operators' native call path and the Python checks take the same calls, with the same result, and refuse alike."""
 import ctypes
 
 import pytest
@@ -142,6 +142,36 @@ def test_both_paths_agree(gpu_device, monkeypatch, name):
                     messages.append(str(error))
             assert messages[0] == messages[1]
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["decode", "indexed", "rope", "prefill", "key_split", "exchange"])
+def test_both_paths_refuse_alike(gpu_device, monkeypatch, name):
+    """Tensors of another device, of another shape (one entry more in the first dimension) and with a base that is not
+    aligned, one at a time: both paths take the call or refuse it with the same words. All of them are refused on the
+    host where a kernel could not take them."""
+    call, args, _ = calls(gpu_device)[name]
+    native, refused = cuda_runtime.fast_call(), 0
+    for index, tensor in enumerate(args):
+        if not isinstance(tensor, torch.Tensor) or not tensor.numel():
+            continue
+        shifted = torch.empty(tensor.numel() + 1, dtype=tensor.dtype, device=gpu_device)[1:].view(tensor.shape)
+        longer = torch.cat([tensor, tensor[:1]])
+        for wrong in (tensor.cpu(), longer, shifted.copy_(tensor)):
+            messages = []
+            for path in (native, None):
+                monkeypatch.setattr(cuda_runtime, "fast_call", lambda: path)
+                changed = list(args)
+                changed[index] = wrong
+                try:
+                    call(*changed)
+                    messages.append("")
+                except RuntimeError as error:
+                    messages.append(str(error))
+            assert messages[0] == messages[1], (index, messages)
+            refused += messages[0] != ""
+        torch.cuda.synchronize()
+    assert refused >= 2 * 5  # at least the five leading tensors, on another device and of another shape
 
 
 @pytest.mark.gpu
