@@ -106,7 +106,9 @@ int tc_prefill_resources(int device, const int64_t q_strides[3], const int64_t k
  * of 2 to 64 sequences may then be split on the device by the lengths it finds there: spec[1] and spec[2] are the
  * workspace that this takes, larger than spec[0] splits need and not zero where spec[0] == 1 (the partials and, behind
  * the LSEs, 4 elements of ticket per (sequence, KV head)); it needs no initial value. With a workspace that holds
- * spec[0] splits only, those are what the call uses.
+ * spec[0] splits only, those are what the call uses. Split by length, a sequence's shares follow from the lengths of the
+ * whole batch, so the order of its sums, and with it the last bits of O and LSE, may change with its neighbours' lengths
+ * (the caches never do); a positive num_splits cuts every sequence by its own length alone.
  */
 int tc_decode_workspace_spec(int device, int64_t batch, int64_t capacity, int64_t kv_heads, int64_t num_splits,
                              int64_t mapping, int append, int64_t spec[3]);
@@ -134,7 +136,8 @@ int tc_decode_forward_out(int device, void* stream, const void* q, void* kcache,
  * old_lengths[b], old_lengths itself (and, where used, index tables). The launch uses programmatic dependent
  * launch; with the flag the length read and the K/V stream start while that preceding kernel is still
  * finishing (the first tiles into the shared-memory ring, the others as prefetches into L2), and only q, knew,
- * vnew and all writes wait for it. Typical cases: the preceding kernel is the projection that produces q / knew
+ * vnew and all writes wait for it (a launch split by length takes one CTA slot per SM under the flag, so on an SM its
+ * stream starts when the preceding kernel's CTA leaves; measured, even placement is worth more). Typical cases: the preceding kernel is the projection that produces q / knew
  * / vnew, or the decode step of another layer (other caches). TC_DECODE_PREFIX_STABLE is the narrower promise
  * for a preceding kernel that was the previous decode step of the SAME caches: it may have written row
  * old_lengths[b] - 1 and nothing else of the above; then only the tiles that end below that row are fetched

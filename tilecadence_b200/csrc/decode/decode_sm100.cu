@@ -53,7 +53,8 @@ constexpr int ring_period(int a, int b) {
 constexpr int kRingPeriod = ring_period(kStages, kGroups);
 // Registers per thread such that AB_DECODE_CTAS_PER_SM CTAs fit an SM. Registers belong to the SM's quarters, 16 K
 // each, and are allocated per warp in multiples of 8 per thread: the fullest quarter counts (168 for two CTAs of five
-// warps; at 176 only one CTA was resident).
+// warps. As written the kernel takes 168 by itself; other arrangements of the same code took 172 and 180 without the
+// limit, which leaves room for one CTA).
 constexpr int kWarpsPerQuarter = (AB_DECODE_CTAS_PER_SM * kThreads / 32 + 3) / 4;
 constexpr int kMaxRegisters = 16384 / (32 * kWarpsPerQuarter) / 8 * 8;
 constexpr int kGroup = 4;  // query heads per KV head
@@ -199,9 +200,9 @@ __device__ __forceinline__ int visible_rows(const Params& p, int64_t old_len) {
 //   than put one CTA on every SM, kSecondCost and a twelfth of the stream.
 // Lengths of which none outlasts the stream by what a split costs need no search: they are not split.
 // Measured (us, even splits before, by length now): 16 sequences of 500-8000 rows 70.3 -> 41.9, 24 of 300-5000
-// 52.9 -> 33.9, 8 of 200-3333 20.0 -> 14.8. Equal lengths pay for the look at all of them: 8 of 2000 rows 15.3 -> 15.5,
-// 2 of 8192 15.6 -> 15.9; a search, where lengths are close, cost 0.9 at four of about 2000 (11.9 against 11.0).
-// Out of line: inlined ahead of the first load it cost every launch 0.1 to 0.2.
+// 52.9 -> 33.9, 8 of 200-3333 20.2 -> 14.8. Equal lengths pay for the look at all of them: 8 of 2000 rows 15.3 -> 15.5,
+// 2 of 8192 15.8 -> 15.9; a search, where lengths are close, cost 1.0 at four of about 2000 (12.0 against 11.0).
+// Out of line: inlined ahead of the first load it cost every launch 0.1.
 struct Share {
     int b, split, splits, first;  // first: slot of the sequence's first share; splits == 0: nothing to do
     int old_length;
@@ -356,8 +357,8 @@ __device__ unsigned int g_trace_ctas;
 #endif
 
 // kByLength: see plan_share. A launch with the same number of splits for every sequence is an instance of its own, so
-// that it pays nothing for the choice: one sequence of 8192 rows in a chain of layers 18.9 -> 17.8 us a layer, under the
-// cache promise 11.5 -> 10.7.
+// that it pays nothing for the choice: one sequence of 8192 rows in a chain of layers 18.7 -> 17.9 us a layer, under the
+// cache promise 11.5 -> 11.0.
 template <bool kHandoff, bool kPeer, bool kByLength>
 __global__ void __maxnreg__(kMaxRegisters)
 decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
@@ -509,7 +510,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
             return true;
         };
         if (!p.block_table) {
-            // (lane 0, not an elected lane: 10.7 against 11.2 us for one sequence of 8192 rows under the promise)
+            // (lane 0, not an elected lane: 0.4 us less for one sequence of 8192 rows under the promise)
             if (lane == 0) {
                 const int ring_early = early_tiles < kStages ? early_tiles : kStages;
                 bool ok = true;
