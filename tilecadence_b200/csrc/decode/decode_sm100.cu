@@ -202,7 +202,6 @@ __device__ __forceinline__ int visible_rows(const Params& p, int64_t old_len) {
 // Measured (us, even splits before, by length now): 16 sequences of 500-8000 rows 70.3 -> 41.9, 24 of 300-5000
 // 52.9 -> 33.9, 8 of 200-3333 20.2 -> 14.8. Equal lengths pay for the look at all of them: 8 of 2000 rows 15.3 -> 15.5,
 // 2 of 8192 15.8 -> 15.9; a search, where lengths are close, cost 1.0 at four of about 2000 (12.0 against 11.0).
-// Out of line: inlined ahead of the first load it cost every launch 0.1.
 struct Share {
     int b, split, splits, first;  // first: slot of the sequence's first share; splits == 0: nothing to do
     int old_length;
@@ -214,7 +213,7 @@ struct PlanInput {
 };
 // length0, length1: of this lane's sequences, `lane` and `lane + 32`; lanes beyond the batch repeat its last one (for the
 // extremes) with a weight of 0 (for the sums).
-__device__ __noinline__ void plan_share(const PlanInput p, int length0, int length1, int slot, int lane, Share* out) {
+__device__ __forceinline__ void plan_share(const PlanInput& p, int length0, int length1, int slot, int lane, Share* out) {
     constexpr uint32_t kAll = 0xffffffffu;
     const int last = p.batch - 1;
     const int old0 = max(length0, 0), old1 = max(length1, 0);
@@ -277,6 +276,9 @@ __device__ __noinline__ void plan_share(const PlanInput p, int length0, int leng
     const int found0 = __shfl_sync(kAll, old0, share.b & 31), found1 = __shfl_sync(kAll, old1, share.b & 31);
     share.old_length = share.b < 32 ? found0 : found1;
     if (lane == 0) *out = share;
+}
+__device__ __noinline__ void plan_share_far(const PlanInput p, int length0, int length1, int slot, int lane, Share* out) {
+    plan_share(p, length0, length1, slot, lane, out);
 }
 
 // Ticket of a launch split by length, for one thread of each CTA. Whoever found the word unarmed tries to arm it with a
@@ -356,10 +358,17 @@ __device__ unsigned int g_trace_ctas;
 #define TC_TRACE_POINT(slot) do { } while (0)
 #endif
 
-// kByLength: see plan_share. A launch with the same number of splits for every sequence is an instance of its own, so
-// that it pays nothing for the choice: one sequence of 8192 rows in a chain of layers 18.7 -> 17.9 us a layer, under the
-// cache promise 11.5 -> 11.0.
-template <bool kHandoff, bool kPeer, bool kByLength>
+// How a launch cuts its sequences, an instance of the kernel each:
+// kEven: the same number of splits for every sequence. It pays nothing for the choice (one sequence of 8192 rows in a
+//   chain of layers 18.7 -> 17.9 us a layer, under the cache promise 11.5 -> 11.0).
+// kClose: by length where two or more even splits are usual. Lengths are mostly close enough for those, so every warp
+//   looks for itself and the plan is out of line.
+// kPlanned: by length where a sequence usually is one share. One warp looks, the others take its answer, the plan is in
+//   line, an elected lane issues: against kClose 32 ragged sequences up to 3000 rows 35.9 -> 35.1 us, 16 up to 4000 under
+//   the cache promise 24.0 -> 23.6. The other way round four equal sequences of 4096 rows took 16.2 for 16.0, and with the
+//   plan in line ahead of the first load 0.1 more.
+enum Cut { kEven, kClose, kPlanned };
+template <bool kHandoff, bool kPeer, Cut kCut>
 __global__ void __maxnreg__(kMaxRegisters)
 decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                       const DecodeParams p) {
@@ -375,6 +384,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
 
     // A launch that splits by length has its slots in blockIdx.x and blockIdx.z, so that equal lengths give every CTA
     // the place it has in a launch with even splits, and a coarse cut occupies the first CTAs of the grid, one per SM.
+    constexpr bool kByLength = kCut != kEven;
     const int kvh = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q_heads = p.kv_heads * kGroup;
@@ -408,37 +418,45 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     Share share{int(blockIdx.z), int(blockIdx.x), p.splits, 0, 0};
     __shared__ Share planned;  // split by length: the CTA's share, as the producer warp saw it
     if constexpr (kByLength) {
-        // Every warp looks at all lengths and knows without waiting for another whether they are close; if so its share
-        // is its place in the grid (every CTA decides alike). If not, the producer warp plans for the CTA. Which warps
-        // leave and which meet at the barriers of the epilogue follows from `planned` alone: a broken promise may show
-        // the warps different lengths, and none must wait for a warp that has left (waits for tiles end by themselves).
-        // (All warps taking the producer's answer instead: 0.2 to 0.4 us more; a barrier that also votes: 0.6.)
-        const int last = p.batch - 1;
-        share.b = share.b < last ? share.b : last;
-        share.old_length = p.old_lengths[share.b];
-        // (lanes beyond the batch repeat its last sequence)
-        const int32_t old0 = p.old_lengths[lane < last ? lane : last];
-        const int32_t old1 = p.batch > 32 ? p.old_lengths[lane + 32 < last ? lane + 32 : last] : old0;
-        const uint32_t apart = uint32_t(__reduce_max_sync(0xffffffffu, max(old0, old1))) -
-                               uint32_t(__reduce_min_sync(0xffffffffu, min(old0, old1)));
-        const bool close = apart <= uint32_t(2 * kTileN * p.splits);
-        share.old_length = max(share.old_length, 0);
-        share.first = share.b * p.splits;
-        if (int(blockIdx.z) > last) share.splits = 0;
-        if (warp == kConsumerWarps) {
-            if (!close)
-                plan_share({p.shard_start, p.batch, p.capacity, p.kv_heads, p.append, p.plan_slots, p.plan_even}, old0, old1,
-                           int(blockIdx.x + blockIdx.z * gridDim.x), lane, &planned);
-            else if (lane == 0)
-                planned = share;
+        // If the shares of even splits differ by two tiles at most, a CTA's share is its place in the grid (every CTA
+        // decides alike); otherwise the producer warp plans for its CTA. kClose: every warp sees by itself which it is and
+        // goes on from its own registers if the lengths are close (all of them taking the producer's answer instead: 0.2 to
+        // 0.4 us more; a barrier that also votes: 0.6). Which warps leave and which meet at the barriers of the epilogue
+        // still follows from `planned` alone: a broken promise may show the warps different lengths, and none must wait
+        // for a warp that has left (waits for tiles end by themselves).
+        bool close = false;
+        if (kCut == kClose || warp == kConsumerWarps) {
+            const int last = p.batch - 1;
+            share.b = share.b < last ? share.b : last;
+            share.old_length = p.old_lengths[share.b];
+            // (lanes beyond the batch repeat its last sequence)
+            const int32_t old0 = p.old_lengths[lane < last ? lane : last];
+            const int32_t old1 = p.batch > 32 ? p.old_lengths[lane + 32 < last ? lane + 32 : last] : old0;
+            const uint32_t apart = uint32_t(__reduce_max_sync(0xffffffffu, max(old0, old1))) -
+                                   uint32_t(__reduce_min_sync(0xffffffffu, min(old0, old1)));
+            close = apart <= uint32_t(2 * kTileN * p.splits);
+            share.old_length = max(share.old_length, 0);
+            share.first = share.b * p.splits;
+            if (int(blockIdx.z) > last) share.splits = 0;
+            if (warp == kConsumerWarps) {
+                const PlanInput input{p.shard_start, p.batch, p.capacity, p.kv_heads, p.append, p.plan_slots, p.plan_even};
+                const int slot = int(blockIdx.x + blockIdx.z * gridDim.x);
+                if (close) {
+                    if (lane == 0) planned = share;
+                } else if (kCut == kClose) {
+                    plan_share_far(input, old0, old1, slot, lane, &planned);
+                } else {
+                    plan_share(input, old0, old1, slot, lane, &planned);
+                }
+            }
         }
         __syncthreads();
-        if (!close) share = planned;
-        if (share.splits == 0 && planned.splits == 0) return;  // more slots than shares
+        if (kCut == kPlanned || !close) share = planned;
+        if (share.splits == 0 && (kCut == kPlanned || planned.splits == 0)) return;  // more slots than shares
     }
     const int64_t old_len = kByLength ? share.old_length : old_length(p, share.b);
-    const int b = share.b, split = share.split, splits = kByLength ? max(share.splits, 1) : share.splits;
-    const int n_valid = kByLength && share.splits == 0 ? 0 : visible_rows(p, old_len);
+    const int b = share.b, split = share.split, splits = kCut == kClose ? max(share.splits, 1) : share.splits;
+    const int n_valid = kCut == kClose && share.splits == 0 ? 0 : visible_rows(p, old_len);
     const int64_t append_local = old_len - p.shard_start;
     const bool do_append = p.append && append_local >= 0 && append_local < p.capacity;
     const int append_row = do_append ? int(append_local) : -1;
@@ -511,7 +529,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         };
         if (!p.block_table) {
             // (lane 0, not an elected lane: 0.4 us less for one sequence of 8192 rows under the promise)
-            if (lane == 0) {
+            if (kCut == kPlanned ? tc::elect_one() : lane == 0) {
                 const int ring_early = early_tiles < kStages ? early_tiles : kStages;
                 bool ok = true;
                 int it = 0;
@@ -746,7 +764,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     // Quad-partial row sums become full sums; each warp parks its partial in the K rows it owns in its
     // group's terminal stage (nobody else reads those rows: the group is done with them and the other
     // group never reads that stage again), then one barrier releases the stages.
-    if constexpr (kByLength) {
+    if constexpr (kCut == kClose) {
         share = planned;  // read again here: held in registers over the key loop it cost more
         if (share.splits == 0) return;
     }
@@ -1075,9 +1093,9 @@ int check_geometry(int device, int64_t batch, int64_t capacity, int64_t kv_heads
     return TC_OK;
 }
 
-template <bool kHandoff, bool kPeer, bool kByLength>
+template <bool kHandoff, bool kPeer, Cut kCut>
 int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, bool spread, cudaStream_t stream) {
-    auto kernel = &decode_splitkv_kernel<kHandoff, kPeer, kByLength>;
+    auto kernel = &decode_splitkv_kernel<kHandoff, kPeer, kCut>;
     constexpr int shared = shared_bytes(kHandoff);
     static thread_local int configured_device = -1;
     static thread_local int64_t resident_ctas = 0;
@@ -1095,7 +1113,7 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
         configured_device = device;
     }
     cudaLaunchConfig_t config{};
-    const int depth = kByLength ? (p.plan_slots + p.splits - 1) / p.splits : p.batch;
+    const int depth = kCut != kEven ? (p.plan_slots + p.splits - 1) / p.splits : p.batch;
     // Every CTA of the grid must be resident at once: a CTA that waits for another rank holds its slot, and the CTAs it
     // indirectly waits for on that rank must never queue behind waiters. What fits is asked of this very kernel.
     if (kPeer)
@@ -1115,12 +1133,19 @@ int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams&
     return TC_OK;
 }
 
+Cut cut_of(int64_t slots, int splits) { return slots == 0 ? kEven : splits > 1 ? kClose : kPlanned; }
+
 template <bool kPeer>
 int launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, bool handoff, bool spread, void* stream) {
     const auto s = static_cast<cudaStream_t>(stream);
-    if (p.plan_slots > 0)
-        return handoff ? launch<true, kPeer, true>(kmap, vmap, p, spread, s) : launch<false, kPeer, true>(kmap, vmap, p, spread, s);
-    return handoff ? launch<true, kPeer, false>(kmap, vmap, p, false, s) : launch<false, kPeer, false>(kmap, vmap, p, false, s);
+    switch (cut_of(p.plan_slots, p.splits)) {
+        case kClose:
+            return handoff ? launch<true, kPeer, kClose>(kmap, vmap, p, spread, s) : launch<false, kPeer, kClose>(kmap, vmap, p, spread, s);
+        case kPlanned:
+            return handoff ? launch<true, kPeer, kPlanned>(kmap, vmap, p, spread, s) : launch<false, kPeer, kPlanned>(kmap, vmap, p, spread, s);
+        default:
+            return handoff ? launch<true, kPeer, kEven>(kmap, vmap, p, false, s) : launch<false, kPeer, kEven>(kmap, vmap, p, false, s);
+    }
 }
 
 struct PeerArgs {
@@ -1487,8 +1512,13 @@ int tc_decode_resources(int device, int64_t batch, int64_t capacity, int64_t kv_
     const int64_t header[12] = {splits, kGroup, kv_heads, kGroup, 1, slots > 0 ? slots * kv_heads : batch * kv_heads * splits,
                                 o_elems > 0 ? batch * kv_heads : 0, o_elems, lse_elems, kGroup, kTileN, 1};
     for (int i = 0; i < 12; ++i) values[i] = header[i];
-    const auto kernel = slots > 0 ? (mapping == 1 ? &decode_splitkv_kernel<true, false, true> : &decode_splitkv_kernel<false, false, true>)
-                                  : (mapping == 1 ? &decode_splitkv_kernel<true, false, false> : &decode_splitkv_kernel<false, false, false>);
+    const Cut cut = cut_of(slots, splits);
+    const auto kernel = mapping == 1 ? (cut == kEven    ? &decode_splitkv_kernel<true, false, kEven>
+                                        : cut == kClose ? &decode_splitkv_kernel<true, false, kClose>
+                                                        : &decode_splitkv_kernel<true, false, kPlanned>)
+                                     : (cut == kEven    ? &decode_splitkv_kernel<false, false, kEven>
+                                        : cut == kClose ? &decode_splitkv_kernel<false, false, kClose>
+                                                        : &decode_splitkv_kernel<false, false, kPlanned>);
     const bool spread = one_per_sm(info, slots, splits, batch, capacity, kv_heads, 0);
     status = tc::kernel_resources(kernel, kThreads, spread ? kSpreadShared : shared_bytes(mapping == 1), values + 12);
     if (status != TC_OK) return status;
