@@ -729,3 +729,34 @@ def test_steps_split_by_length_may_overlap_under_a_promise(ops, gpu_device, batc
 def test_rotary_embedding_in_a_launch_split_by_length(ops, gpu_device):
     lengths = [4095, 200, 3000, 64, 0, 1500, 777, 2048]
     test_rotary_embedding_inside_the_launch(ops, gpu_device, 8, 4096, lengths, 0)
+
+
+@pytest.mark.parametrize("batch,length,lengths", [
+    (4, 2560, [7600, 100, 2559, 5121]),                               # two shards that some sequences never reach
+    (12, 1024, [3000, 5, 1024, 1023, 2047, 64, 700, 0, 1500, 2048, 3071, 333]),
+])
+def test_shards_split_by_length(ops, gpu_device, batch, length, lengths):
+    """Partial results of three shards of a longer cache, each launch split by the lengths it sees of its shard (none of
+    some sequences, all of others): combined they are the oracle's result, and the shard that holds the new row, only
+    that one, appends it."""
+    shards, capacity, device = 3, 3 * length, gpu_device
+    q, kcache, vcache, knew, vnew = make_case(81, batch, capacity, fill=lengths)
+    old = torch.tensor(lengths, dtype=torch.int32)
+    want_o, want_lse, want_k, want_v = oracle.decode_step(q, kcache, vcache, knew, vnew, old)
+    dq, dkn, dvn, dold = (t.to(device) for t in (q, knew, vnew, old))
+    part_o = torch.full((shards, batch * 32, 128), float("nan"), device=device)
+    part_lse = torch.full((shards, batch * 32), float("nan"), device=device)
+    for s in range(shards):
+        rows = slice(s * length, (s + 1) * length)
+        dk, dv = kcache[:, rows].contiguous().to(device), vcache[:, rows].contiguous().to(device)
+        spec = ops.workspace_spec(dq, dk, dold, 0, 1, True)
+        assert spec[1:] != ops.workspace_spec(dq, dk, dold, spec[0], 1, True)[1:]  # split by length
+        ws = [torch.full((n,), float("nan"), device=device) for n in spec[1:3]]
+        ops.partial_out(dq, dk, dv, dkn, dvn, dold, part_o[s], part_lse[s], *ws, 0, 1, True, s * length)
+        torch.cuda.synchronize()
+        assert torch.equal(bits(dk.cpu()), bits(want_k[:, rows])) and torch.equal(bits(dv.cpu()), bits(want_v[:, rows]))
+    out, lse = torch.empty_like(dq), torch.empty((batch, 32, 1), device=device)
+    ops.combine_partials(part_o, part_lse, out, lse)
+    torch.cuda.synchronize()
+    assert ops.library.device_status(device.index) == 0
+    oracle.check_outputs(out.cpu(), lse.cpu(), want_o, want_lse)
